@@ -75,6 +75,13 @@ struct SysView {
   const double* pot_site_pos;        // [3*npotsites]
   const int32_t* pot_site_type;
   int32_t num_pot_sites;
+  // images C' = C + T of the potential sites around each atom A, grouped by
+  // [atom][potential type], ordered by shells of |C' - A| within a group:
+  // every image a third-centre sum of an alpha pair on A can reach
+  const int32_t* img_start;          // [natoms*num_pot_types + 1]
+  const double4_16a* img_d;              // C' - A (x, y, z, 0)
+  const float4* img_hi;              // C' - A rounded; w: below |C' - A|, its shell
+  const float4* img_lo;              // the rounding's remainder
   const double* elem_alpha;          // [nelem*OLC_MAX_ALPHAS]
   const double* elem_nuc_alpha;      // [nelem]
   const double* elem_pot_alpha;      // [nelem*OLC_MAX_POT_ALPHAS]

@@ -24,7 +24,7 @@ namespace olc {
 // ---------------------------------------------------------------------------
 // stage 1: primitive kernels
 // ---------------------------------------------------------------------------
-template <int OP, int MODE>
+template <int OP, bool FAR32>
 int launch_class(olc_context* ctx, int cls, const double* coeffs, int ep_type, int ep_alpha,
                  bool accumulate) {
   const ItemLists& it = ctx->items;
@@ -38,7 +38,7 @@ int launch_class(olc_context* ctx, int cls, const double* coeffs, int ep_type, i
   a.ep_type = ep_type;
   a.ep_alpha = ep_alpha;
   if (a.n == 0) return OLC_OK;
-  const dim3 block(128), grid((a.n + 127) / 128);
+  const dim3 block(kThirdThreads), grid((a.n + kThirdThreads - 1) / kThirdThreads);
   StageScope scope(ctx, OLC_STAGE_PRIMITIVES);
   const int l1 = cls / (kMaxL + 1), l2 = cls % (kMaxL + 1);
   if (l1 == 3 || l2 == 3) {
@@ -47,18 +47,23 @@ int launch_class(olc_context* ctx, int cls, const double* coeffs, int ep_type, i
       case OLC_OP_KINETIC: return launch_prim_f_kinetic(ctx->stream, ctx->view, a, l1, l2, grid, block);
       case OLC_OP_MASSVEL: return launch_prim_f_massvel(ctx->stream, ctx->view, a, l1, l2, grid, block);
       case OLC_OP_NUCLEAR: return launch_prim_f_nuclear(ctx->stream, ctx->view, a, l1, l2, grid, block);
-      default: return launch_prim_f_elecpot(ctx->stream, ctx->view, a, l1, l2, MODE, grid, block);
+      default: return launch_prim_f_elecpot(ctx->stream, ctx->view, a, l1, l2, FAR32, grid, block);
     }
   }
   switch (l1 * 3 + l2) {
-#define OLC_CASE(c, l1, l2) \
-  case c: prim_kernel<OP, l1, l2, MODE><<<grid, block, 0, ctx->stream>>>(ctx->view, a); break;
+#define OLC_CASE(c, l1, l2)                                                                   \
+  case c:                                                                                     \
+    if constexpr (OP == OLC_OP_NUCLEAR || OP == OLC_OP_ELECPOT)                               \
+      third_centre_kernel<OP, l1, l2, FAR32><<<grid, block, 0, ctx->stream>>>(ctx->view, a);  \
+    else                                                                                      \
+      prim_kernel<OP, l1, l2><<<grid, block, 0, ctx->stream>>>(ctx->view, a);                 \
+    break;
     OLC_CASE(0, 0, 0) OLC_CASE(1, 0, 1) OLC_CASE(2, 0, 2)
     OLC_CASE(3, 1, 0) OLC_CASE(4, 1, 1) OLC_CASE(5, 1, 2)
     OLC_CASE(6, 2, 0) OLC_CASE(7, 2, 1) OLC_CASE(8, 2, 2)
 #undef OLC_CASE
   }
-  return cuda_check(cudaGetLastError(), "prim_kernel launch");
+  return cuda_check(cudaGetLastError(), "primitive kernel launch");
 }
 
 int run_primitives(olc_context* ctx, int op, int term, const double* coeffs, int precision,
@@ -79,17 +84,13 @@ int run_primitives(olc_context* ctx, int op, int term, const double* coeffs, int
   for (int cls = 0; cls < kNumClasses; ++cls) {
     int st = 0;
     switch (op) {
-      case OLC_OP_OVERLAP: st = launch_class<OLC_OP_OVERLAP, 0>(ctx, cls, nullptr, -1, 0, accumulate); break;
-      case OLC_OP_KINETIC: st = launch_class<OLC_OP_KINETIC, 0>(ctx, cls, nullptr, -1, 0, accumulate); break;
-      case OLC_OP_MASSVEL: st = launch_class<OLC_OP_MASSVEL, 0>(ctx, cls, nullptr, -1, 0, accumulate); break;
-      case OLC_OP_NUCLEAR: st = launch_class<OLC_OP_NUCLEAR, 0>(ctx, cls, nullptr, -1, 0, accumulate); break;
+      case OLC_OP_OVERLAP: st = launch_class<OLC_OP_OVERLAP, false>(ctx, cls, nullptr, -1, 0, accumulate); break;
+      case OLC_OP_KINETIC: st = launch_class<OLC_OP_KINETIC, false>(ctx, cls, nullptr, -1, 0, accumulate); break;
+      case OLC_OP_MASSVEL: st = launch_class<OLC_OP_MASSVEL, false>(ctx, cls, nullptr, -1, 0, accumulate); break;
+      case OLC_OP_NUCLEAR: st = launch_class<OLC_OP_NUCLEAR, false>(ctx, cls, nullptr, -1, 0, accumulate); break;
       case OLC_OP_ELECPOT:
-        if (far32) {
-          st = launch_class<OLC_OP_ELECPOT, 1>(ctx, cls, coeffs, ep_type, ep_alpha, accumulate);
-          if (!st) st = launch_class<OLC_OP_ELECPOT, 2>(ctx, cls, coeffs, ep_type, ep_alpha, true);
-        } else {
-          st = launch_class<OLC_OP_ELECPOT, 0>(ctx, cls, coeffs, ep_type, ep_alpha, accumulate);
-        }
+        st = far32 ? launch_class<OLC_OP_ELECPOT, true>(ctx, cls, coeffs, ep_type, ep_alpha, accumulate)
+                   : launch_class<OLC_OP_ELECPOT, false>(ctx, cls, coeffs, ep_type, ep_alpha, accumulate);
         break;
       default: return fail(OLC_ERR_ARG, "unknown integral operator");
     }

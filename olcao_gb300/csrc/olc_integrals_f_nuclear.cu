@@ -7,7 +7,7 @@ namespace olc {
 int launch_prim_f_nuclear(cudaStream_t st, const SysView& v, const PrimArgs& a, int l1, int l2, dim3 g, dim3 b) {
   switch (l1 * 4 + l2) {
 #define OLC_FCASE(L1, L2) \
-  case L1 * 4 + L2: prim_kernel<OLC_OP_NUCLEAR, L1, L2, 0><<<g, b, 0, st>>>(v, a); break;
+  case L1 * 4 + L2: third_centre_kernel<OLC_OP_NUCLEAR, L1, L2, false><<<g, b, 0, st>>>(v, a); break;
     OLC_FCASE(0, 3) OLC_FCASE(1, 3) OLC_FCASE(2, 3) OLC_FCASE(3, 0) OLC_FCASE(3, 1) OLC_FCASE(3, 2) OLC_FCASE(3, 3)
 #undef OLC_FCASE
     default: return fail(OLC_ERR_ARG, "not an f class");

@@ -4,8 +4,6 @@
 // recurrences are large).
 #pragma once
 
-#include <type_traits>
-
 #include "olc_common.h"
 #include "olc_primitives.cuh"
 
@@ -24,30 +22,14 @@ __device__ __forceinline__ double alpha_dist(const SysView& v, int a1, int a2, i
   return v.log_thresh / ak / (al / (al + ak));
 }
 
-// Reduce v by the lattice vector obtained from rounding its fractional
-// coordinates (the first step of findLatticeVector, lattice.f90:777-793).
-__device__ __forceinline__ void round_reduce(const SysView& v, const double* in, double* out) {
-  double L[3] = {0.0, 0.0, 0.0};
-#pragma unroll
-  for (int i = 0; i < 3; ++i) {
-    const double f = in[0] * v.inv_real[i * 3] + in[1] * v.inv_real[i * 3 + 1] +
-                     in[2] * v.inv_real[i * 3 + 2];
-    double r = floor(fabs(f) + 0.5);
-    if (f < 0.0) r = -r;
-#pragma unroll
-    for (int c = 0; c < 3; ++c) L[c] += v.real_vec[i * 3 + c] * r;
-  }
-#pragma unroll
-  for (int c = 0; c < 3; ++c) out[c] = in[c] - L[c];
-}
-
 struct ItemGeom {
   double A[3], B[3];
   double a1, a2, sep;
   int e1, e2, ia1, ia2;
 };
 
-__device__ __forceinline__ void load_item(const SysView& v, int task, int ab, ItemGeom& g) {
+// Returns the atom A of the item.
+__device__ __forceinline__ int load_item(const SysView& v, int task, int ab, ItemGeom& g) {
   const DevTask tk = v.tasks[task];
   const DevPair p = v.pairs[tk.pair];
   const DevType& t1 = v.types[v.site_type[p.i]];
@@ -64,31 +46,7 @@ __device__ __forceinline__ void load_item(const SysView& v, int task, int ab, It
   g.e1 = t1.element;
   g.e2 = t2.element;
   g.sep = tk.sep;
-}
-
-// Visit every lattice image C' = C + T of a site with |P - C'|^2 <= tad.
-// The image set equals the reference's {cells of the nearest-origin loop},
-// integrals.F90:2374-2418 / 2533-2594.
-template <class F>
-__device__ __forceinline__ void for_images(const SysView& v, const double* P, const double* C,
-                                           double tad, F&& f) {
-  double d[3] = {P[0] - C[0], P[1] - C[1], P[2] - C[2]};
-  double r[3];
-  round_reduce(v, d, r);
-  const double rn = sqrt(r[0] * r[0] + r[1] * r[1] + r[2] * r[2]);
-  const double lim = rn + sqrt(tad);
-  const double lim2 = lim * lim;
-  // base image of C: C + (d - r)
-  const double base[3] = {C[0] + (d[0] - r[0]), C[1] + (d[1] - r[1]), C[2] + (d[2] - r[2])};
-  for (int n = 0; n < v.ncells; ++n) {
-    const double4 cell = reinterpret_cast<const double4*>(v.cells)[n];
-    if (cell.w > lim2) break;
-    const double x = r[0] - cell.x, y = r[1] - cell.y, z = r[2] - cell.z;
-    const double d2 = x * x + y * y + z * z;
-    if (d2 > tad) continue;
-    const double Cp[3] = {base[0] + cell.x, base[1] + cell.y, base[2] + cell.z};
-    f(Cp, d2);
-  }
+  return p.i;
 }
 
 // ---------------------------------------------------------------------------
@@ -105,89 +63,217 @@ struct PrimArgs {
   int ep_alpha;             // EP: exponent index of a single term
 };
 
-// MODE 0: every term in FP64.  Mixed precision splits the electronic
-// potential into two passes: MODE 1 the near images (FP64), MODE 2 the images
-// past the far-shell cut (FP32 accumulator), added to the same blocks.
-template <int OP, int L1, int L2, int MODE>
+// Two-centre operators, one thread per item.
+template <int OP, int L1, int L2>
 __global__ void __launch_bounds__(128) prim_kernel(SysView v, PrimArgs a) {
   const int idx = blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= a.n) return;
   constexpr int N1 = ncart(L1), N2 = ncart(L2), NS = nharm(L1) * nharm(L2);
   ItemGeom g;
   load_item(v, a.task[idx], a.ab[idx], g);
-  using R = typename std::conditional<MODE == 2, float, double>::type;
-  R cart[N1 * N2];
+  double cart[N1 * N2];
 #pragma unroll
-  for (int q = 0; q < N1 * N2; ++q) cart[q] = R(0);
-  double scale = 1.0;
+  for (int q = 0; q < N1 * N2; ++q) cart[q] = 0.0;
   if constexpr (OP == OLC_OP_OVERLAP) {
     add_overlap<L1, L2>(g.a1, g.a2, g.A, g.B, 1.0, cart);
   } else if constexpr (OP == OLC_OP_KINETIC) {
     add_kinetic<L1, L2>(g.a1, g.a2, g.A, g.B, 1.0, cart);
-  } else if constexpr (OP == OLC_OP_MASSVEL) {
+  } else {
     // gaussOverlapMV accumulates the primitive with a minus sign
     // (integrals.F90:1228-1236): the mass-velocity term lowers H
     add_massvel<L1, L2>(g.a1, g.a2, g.A, g.B, -1.0, cart);
-  } else {
-    // centre of the alpha-pair overlap (alphaCenter, gaussRelations.f90:122)
-    const double al = elem_alpha(v, g.e1, g.ia1), ak = elem_alpha(v, g.e2, g.ia2);
-    const double cen = al / (al + ak);
-    double P[3];
+  }
+  store_harmonic<L1, L2, double>(cart, a.out + (size_t)idx * NS, a.accumulate != 0, 1.0);
+}
+
+// Third-centre operators (nuclear attraction, electronic potential), one
+// thread per item: the moments about P summed over the images within the
+// reference's radius (the image set of integrals.F90:2374-2418, 2533-2594),
+// then one transformation into the item's Cartesian block.
+//
+// GB300's FP64 pipe issues a warp instruction every 64 cycles per scheduler,
+// so the kernel is bound by the FP64 instructions of the lanes' images.  The
+// images come from the atom's list (SysView::img_*) and are screened in FP32
+// with a margin wider than its rounding; the survivors go to a queue of
+// kQueue entries per thread in shared memory, so that a warp spends FP64
+// instructions on rounds in which every lane has an image left, not on
+// candidates that only one lane accepts; the exact test |P - C'|^2 <= radius^2
+// is repeated in FP64 on them.  Measured on the 64-atom silicon cell's d-d
+// class, one FP64 potential term: 2.0 ms (8.5 ms with a Cartesian block per
+// image and the images found from the cell list); f-f on a two-atom cell:
+// 0.52 ms (2.3 ms); nuclear d-d on the 64-atom cell: 6.0 ms (17.4 ms).
+//
+// FAR32 (mixed precision): images whose suppression is below exp(-kFarRho)
+// are summed in FP32, in a queue and accumulators of their own, in the same
+// pass (all 16 terms of the 64-atom cell's d-d class: 109 ms in two passes
+// of Cartesian blocks before).
+constexpr int kThirdThreads = 128;
+constexpr int kQueue = 16;
+
+template <int OP, int L1, int L2, bool FAR32>
+__global__ void __launch_bounds__(kThirdThreads) third_centre_kernel(SysView v, PrimArgs a) {
+  constexpr int N1 = ncart(L1), N2 = ncart(L2), NS = nharm(L1) * nharm(L2), LT = L1 + L2, NM = nmom(LT);
+  __shared__ int queue[kQueue][kThirdThreads];
+  __shared__ int farq[FAR32 ? kQueue : 1][FAR32 ? kThirdThreads : 1];
+  const int idx = blockIdx.x * kThirdThreads + threadIdx.x, tid = threadIdx.x;
+  const bool live = idx < a.n;
+  ItemGeom g;
+  const int atom = load_item(v, a.task[live ? idx : 0], a.ab[live ? idx : 0], g);
+  const double z = g.a1 + g.a2, iz = 1.0 / z;
+  double PA[3], PB[3], PS[3];
+  // centre of the alpha-pair overlap (alphaCenter, gaussRelations.f90:122):
+  // the screen's centre, the same point unless two types share an element
+  // with different exponents
+  const double al = elem_alpha(v, g.e1, g.ia1), ak = elem_alpha(v, g.e2, g.ia2);
+  const bool same = al == g.a1 && ak == g.a2;
+  const double izs = 1.0 / (al + ak), frac = 1.0 - g.sep / alpha_dist(v, g.ia1, g.ia2, g.e1, g.e2);
+  double d2ab = 0.0, ps2 = 0.0;
 #pragma unroll
-    for (int c = 0; c < 3; ++c) P[c] = cen * (g.A[c] - g.B[c]) + g.B[c];
-    const double frac = 1.0 - g.sep / alpha_dist(v, g.ia1, g.ia2, g.e1, g.e2);
-    const double T = v.log_thresh;
-    if constexpr (OP == OLC_OP_NUCLEAR) {
-      for (int m = 0; m < v.num_pot_sites; ++m) {
-        const DevPotType& pt = v.pot_types[v.pot_site_type[m]];
-        if (pt.nuc_charge < 1.0e-8) continue;
-        const double an = v.elem_nuc_alpha[pt.element];
-        const double tad = frac * (T * (al + ak + an) / (al + ak) / an);
-        const double nz = -pt.nuc_charge, nalpha = pt.nuc_alpha;
-        for_images(v, P, &v.pot_site_pos[3 * m], tad, [&](const double* Cp, double) {
-          add_nuclear<L1, L2>(g.a1, g.a2, nalpha, g.A, g.B, Cp, nz, cart);
-        });
+  for (int c = 0; c < 3; ++c) {
+    const double ab = g.A[c] - g.B[c];
+    PA[c] = -g.a2 * iz * ab;
+    PB[c] = g.a1 * iz * ab;
+    PS[c] = -ak * izs * ab;
+    d2ab += ab * ab;
+    ps2 += PS[c] * PS[c];
+  }
+  const double expAB = exp(-(g.a1 * g.a2 * iz) * d2ab);
+  const float psf[3] = {(float)PS[0], (float)PS[1], (float)PS[2]};
+  const float ap = (float)sqrt(ps2);
+  float pah[3], pal[3];
+  if (FAR32) {
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      pah[c] = (float)PA[c];
+      pal[c] = (float)(PA[c] - (double)pah[c]);
+    }
+  }
+  double E[NM];
+  float Ef[FAR32 ? NM : 1];
+#pragma unroll
+  for (int q = 0; q < NM; ++q) {
+    E[q] = 0.0;
+    if (FAR32) Ef[q] = 0.f;
+  }
+  bool any = false;
+  const double T = v.log_thresh;
+  const int t0 = OP == OLC_OP_NUCLEAR || a.ep_type < 0 ? 0 : a.ep_type;
+  const int t1 = OP == OLC_OP_NUCLEAR || a.ep_type < 0 ? v.num_pot_types : a.ep_type + 1;
+  for (int t = t0; t < t1; ++t) {
+    const DevPotType& pt = v.pot_types[t];
+    if (OP == OLC_OP_NUCLEAR && pt.nuc_charge < 1.0e-8) continue;
+    const int i0 = live ? v.img_start[atom * v.num_pot_types + t] : 0;
+    const int i1 = live ? v.img_start[atom * v.num_pot_types + t + 1] : 0;
+    const int j0 = OP == OLC_OP_NUCLEAR || a.ep_type < 0 ? 0 : a.ep_alpha;
+    const int j1 = OP == OLC_OP_NUCLEAR ? 1 : a.ep_type < 0 ? pt.num_alphas : a.ep_alpha + 1;
+    for (int j = j0; j < j1; ++j) {
+      const double an = OP == OLC_OP_NUCLEAR ? v.elem_nuc_alpha[pt.element]
+                                             : v.elem_pot_alpha[pt.element * OLC_MAX_POT_ALPHAS + j];
+      const double tad = frac * (T * (al + ak + an) * izs / an);
+      const double a3 = OP == OLC_OP_NUCLEAR ? pt.nuc_alpha : pt.alphas[j];
+      const double z3 = z + a3, iz3 = 1.0 / z3, u = a3 * iz3, rho = z * u, h = 0.5 * iz3;
+      double pref;      // of the moments, the image's exponential apart
+      if (OP == OLC_OP_NUCLEAR) {
+        pref = -pt.nuc_charge * 2.0 * (kPi * iz3) * expAB;
+      } else {
+        const double w = a.coeffs ? a.coeffs[pt.cumul_alpha + j] : 1.0, r = kPi * iz3;
+        pref = w * r * sqrt(r) * expAB;
       }
-    } else {  // electronic potential: single term or sum_j c_j V_j
-      double d2 = 0.0;
-#pragma unroll
-      for (int c = 0; c < 3; ++c) d2 += (g.A[c] - g.B[c]) * (g.A[c] - g.B[c]);
-      const double expAB = exp(-(g.a1 * g.a2 / (g.a1 + g.a2)) * d2);
-      const int t0 = a.ep_type < 0 ? 0 : a.ep_type;
-      const int t1 = a.ep_type < 0 ? v.num_pot_types : a.ep_type + 1;
-      for (int t = t0; t < t1; ++t) {
-        const DevPotType& pt = v.pot_types[t];
-        const double* pe = &v.elem_pot_alpha[pt.element * OLC_MAX_POT_ALPHAS];
-        const int j0 = a.ep_type < 0 ? 0 : a.ep_alpha;
-        const int j1 = a.ep_type < 0 ? pt.num_alphas : a.ep_alpha + 1;
-        // largest radius first: alphaPotDist decreases with the exponent
-        const double tad0 = frac * (T * (al + ak + pe[j0]) / (al + ak) / pe[j0]);
-        for (int m = 0; m < pt.multiplicity; ++m) {
-          const double* C = &v.pot_site_pos[3 * (pt.first_site + m)];
-          for_images(v, P, C, tad0, [&](const double* Cp, double dd) {
-            for (int j = j0; j < j1; ++j) {
-              const double tad = frac * (T * (al + ak + pe[j]) / (al + ak) / pe[j]);
-              if (dd > tad) break;
-              const double w = a.coeffs ? a.coeffs[pt.cumul_alpha + j] : 1.0;
-              if constexpr (MODE == 0) {
-                add_elec3c<L1, L2, double>(g.a1, g.a2, pt.alphas[j], g.A, g.B, Cp, expAB, w, cart);
-              } else {
-                const double rho = elec3c_rho(g.a1, g.a2, pt.alphas[j], g.A, g.B, Cp);
-                if constexpr (MODE == 1) {
-                  if (rho <= kFarRho)
-                    add_elec3c<L1, L2, double>(g.a1, g.a2, pt.alphas[j], g.A, g.B, Cp, expAB, w, cart);
-                } else {
-                  if (rho > kFarRho)
-                    add_elec3c_f32<L1, L2>(g.a1, g.a2, pt.alphas[j], g.A, g.B, Cp, expAB, w, rho, cart);
-                }
-              }
-            }
-          });
+      // FP32 screen: the largest distance from A, and the radius with a
+      // margin of 1e-5 of that distance squared (FP32 differences of numbers
+      // up to it are good to 1e-6 of it)
+      const float reach = (ap + (float)sqrt(tad)) * 1.00001f;
+      const float near2 = (float)tad + 1e-5f * reach * reach;
+      const float rhoh = (float)rho, rhol = (float)(rho - (double)rhoh);
+      int c = i0;
+      bool more = true;
+      while (more) {
+        int cnt = 0, cntf = 0;
+        while (c < i1 && cnt < kQueue && (!FAR32 || cntf < kQueue)) {
+          const float4 q = v.img_hi[c];
+          if (q.w > reach) {
+            c = i1;
+            break;
+          }
+          const float x = psf[0] - q.x, y = psf[1] - q.y, w = psf[2] - q.z;
+          const float d2 = x * x + y * y + w * w;
+          if (d2 <= near2) {
+            if (FAR32 && rhoh * d2 > (float)kFarRho) farq[cntf++][tid] = c;
+            else queue[cnt++][tid] = c;
+          }
+          ++c;
         }
+        __syncwarp();
+        for (int s = 0; s < cnt; ++s) {
+          const double4_16a D = v.img_d[queue[s][tid]];
+          const double x[3] = {PA[0] - D.x, PA[1] - D.y, PA[2] - D.z};       // P - C'
+          const double d2 = x[0] * x[0] + x[1] * x[1] + x[2] * x[2];
+          double ds = d2;
+          if (!same) {
+            const double y[3] = {PS[0] - D.x, PS[1] - D.y, PS[2] - D.z};
+            ds = y[0] * y[0] + y[1] * y[1] + y[2] * y[2];
+          }
+          if (ds > tad) continue;
+          any = true;
+          const double gp[3] = {-u * x[0], -u * x[1], -u * x[2]};            // G - P
+          const double p = pref * exp(-rho * d2);
+          if constexpr (OP == OLC_OP_NUCLEAR) {
+            const double vz = z * iz3;
+            const double gc[3] = {vz * x[0], vz * x[1], vz * x[2]};          // G - C'
+            double F[LT + 1];
+            boys_reference<LT>(z * vz * d2, F);
+            add_nuclear_moments<LT>(gp, gc, h, p, F, E);
+          } else {
+            add_moments<LT, double>(gp, h, p, E);
+          }
+        }
+        if constexpr (FAR32) {
+          const float uf = (float)u, hf = (float)h, prf = (float)pref;
+          for (int s = 0; s < cntf; ++s) {
+            // |P - C'|^2 and rho |P - C'|^2 as FP32 pairs: the exponent keeps
+            // its relative accuracy of about 1e-12 where FP32 alone would lose
+            // 22..37 times 1e-7 of the exponential
+            const int ci = farq[s][tid];
+            const float4 qh = v.img_hi[ci], ql = v.img_lo[ci];
+            float x[3], xl[3], g3[3];
+            pair_sub(pah[0], pal[0], qh.x, ql.x, x[0], xl[0]);
+            pair_sub(pah[1], pal[1], qh.y, ql.y, x[1], xl[1]);
+            pair_sub(pah[2], pal[2], qh.z, ql.z, x[2], xl[2]);
+            float sq[3], se = 0.f;
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+              sq[d] = __fmul_rn(x[d], x[d]);
+              se += __fmaf_rn(x[d], x[d], -sq[d]) + 2.f * x[d] * xl[d];
+              g3[d] = -uf * x[d];
+            }
+            float s1, e1, s2, e2;
+            two_sum(sq[0], sq[1], s1, e1);
+            two_sum(s1, sq[2], s2, e2);
+            se += e1 + e2;
+            const float eh = __fmul_rn(rhoh, s2);
+            const float el = __fmaf_rn(rhoh, s2, -eh) + rhol * s2 + rhoh * se;
+            add_moments<LT, float>(g3, hf, prf * expf(-eh) * (1.f - el), Ef);
+            any = true;
+          }
+        }
+        more = __any_sync(0xffffffffu, c < i1);
       }
     }
   }
-  store_harmonic<L1, L2, R>(cart, a.out + (size_t)idx * NS, a.accumulate != 0, scale);
+  if (!live) return;
+  double* out = a.out + (size_t)idx * NS;
+  if (!any) {
+    if (!a.accumulate)
+#pragma unroll
+      for (int q = 0; q < NS; ++q) out[q] = 0.0;
+    return;
+  }
+  if (FAR32)
+#pragma unroll
+    for (int q = 0; q < NM; ++q) E[q] += (double)Ef[q];
+  double cart[N1 * N2];
+  moments_to_cart<L1, L2>(E, PA, PB, cart);
+  store_harmonic<L1, L2, double>(cart, out, a.accumulate != 0, 1.0);
 }
 
 // One primitive of explicit inputs (the testing entry olc_primitive_batch).
@@ -216,13 +302,14 @@ __device__ __forceinline__ void prim_one(int kind, const double* in, double* out
 }
 
 
-// f classes (olc_integrals_f*.cu): launches of prim_kernel for the 7 classes
-// with l1 = 3 or l2 = 3, one function per operator; mode as prim_kernel.
+// f classes (olc_integrals_f*.cu): launches of the primitive kernels for the
+// 7 classes with l1 = 3 or l2 = 3, one function per operator; far32 as in
+// third_centre_kernel.
 int launch_prim_f_overlap(cudaStream_t st, const SysView& v, const PrimArgs& a, int l1, int l2, dim3 g, dim3 b);
 int launch_prim_f_kinetic(cudaStream_t st, const SysView& v, const PrimArgs& a, int l1, int l2, dim3 g, dim3 b);
 int launch_prim_f_massvel(cudaStream_t st, const SysView& v, const PrimArgs& a, int l1, int l2, dim3 g, dim3 b);
 int launch_prim_f_nuclear(cudaStream_t st, const SysView& v, const PrimArgs& a, int l1, int l2, dim3 g, dim3 b);
-int launch_prim_f_elecpot(cudaStream_t st, const SysView& v, const PrimArgs& a, int l1, int l2, int mode, dim3 g,
+int launch_prim_f_elecpot(cudaStream_t st, const SysView& v, const PrimArgs& a, int l1, int l2, bool far32, dim3 g,
                           dim3 b);
 // primitive batch entries of the f classes, one per kind (1 overlap,
 // 2 kinetic, 3 nuclear, 4 three-centre, 5 mass velocity, 6-8 momentum x, y,

@@ -135,11 +135,13 @@ __device__ __forceinline__ void add_overlap(double a1, double a2, const double* 
       cart[a * N2 + b] += pref * s[0][cex(a)][cex(b)] * s[1][cey(a)][cey(b)] * s[2][cez(a)][cez(b)];
 }
 
-// Cartesian index of exponents (x, y, z), |e| <= 2, in the order above.
+// Cartesian index of exponents (x, y, z), |e| <= 3, in the order above.
 __host__ __device__ constexpr int cidx(int x, int y, int z) {
   return (x + y + z) == 0 ? 0
          : (x + y + z) == 1 ? (x ? 1 : y ? 2 : 3)
-         : (x == 2 ? 4 : y == 2 ? 5 : z == 2 ? 6 : (x && y) ? 7 : (x && z) ? 8 : 9);
+         : (x + y + z) == 2 ? (x == 2 ? 4 : y == 2 ? 5 : z == 2 ? 6 : (x && y) ? 7 : (x && z) ? 8 : 9)
+         : x == 3 ? 10 : y == 3 ? 11 : z == 3 ? 12
+         : x == 2 ? (y ? 13 : 14) : y == 2 ? (x ? 15 : 16) : z == 2 ? (x ? 17 : 18) : 19;
 }
 __host__ __device__ constexpr int cexp(int c, int i) { return i == 0 ? cex(c) : i == 1 ? cey(c) : cez(c); }
 // last non-zero direction of Cartesian c (the direction the recurrence lowers)
@@ -328,49 +330,136 @@ __device__ __forceinline__ void add_elec3c(double a1, double a2, double a3, cons
       cart[a * N2 + b] += pref * s[0][cex(a)][cex(b)] * s[1][cey(a)][cey(b)] * s[2][cez(a)][cez(b)];
 }
 
-// Far-shell split of add_elec3c.  With rho = z a3 / z3 |P - C|^2 an image
-// enters with the suppression exp(-rho); images past kFarRho (exp(-22) =
-// 2.8e-10) may run in FP32 (GB300's FP32 rate is 64x its FP64 rate).  Their
-// FP32 rounding, 6e-8 of a term that the suppression and the recurrence's
-// polynomial in the image distance (up to 25^4 for d-d at the cut-off
-// radius) keep below ~3e-6 of the block scale, stays near 2e-13 of it.
-constexpr double kFarRho = 22.0;
-
-__device__ __forceinline__ double elec3c_rho(double a1, double a2, double a3, const double* A,
-                                             const double* B, const double* Cc) {
-  const double z = a1 + a2;
-  double pc2 = 0.0;
-#pragma unroll
-  for (int c = 0; c < 3; ++c) {
-    const double P = (a1 * A[c] + a2 * B[c]) / z;
-    pc2 += (P - Cc[c]) * (P - Cc[c]);
-  }
-  return z * a3 / (z + a3) * pc2;
+// ---------------------------------------------------------------------------
+// third-centre sums by moments about the pair centre
+// ---------------------------------------------------------------------------
+// A third-centre operator summed over many images C is, for one Gaussian pair,
+// a linear functional of the polynomials (r - A)^a (r - B)^b times the pair's
+// Gaussian about P.  With y = r - P every such polynomial is a short
+// combination of y^e, |e| <= L1 + L2, whose coefficients depend on P - A and
+// P - B only, so the image loop accumulates the moments E(e) = sum_C <y^e>
+// (35 for d-d instead of 100 Cartesian products, 84 instead of 400 for f-f)
+// and the combination is formed once after it.  P - A and P - B come from
+// A - B directly, without the cancellation of G - A for tight functions.
+__host__ __device__ constexpr int nmom(int LT) { return ncart(LT); }
+// index of y^(x, y, z) among the moments, grouped by x, then y
+__host__ __device__ constexpr int midx(int LT, int x, int y, int z) {
+  return nmom(LT) - (LT - x + 1) * (LT - x + 2) * (LT - x + 3) / 6 + (LT - x + 1) * (LT - x + 2) / 2 -
+         (LT - x - y + 1) * (LT - x - y + 2) / 2 + z;
 }
 
-// add_elec3c for a far image, in FP32 (rho from elec3c_rho).
-template <int L1, int L2>
-__device__ __forceinline__ void add_elec3c_f32(double a1, double a2, double a3, const double* A,
-                                               const double* B, const double* Cc, double expAB,
-                                               double w, double rho, float* cart) {
-  constexpr int N1 = ncart(L1), N2 = ncart(L2);
-  const float iz3 = 1.0f / (float)(a1 + a2 + a3);
-  float s[3][L1 + 1][L2 + 1];
+// E(e) += pref <y^e> for the Gaussian exp(-z3 (y - g)^2) normalised to 1
+// (h = 1 / (2 z3)): s[i+1] = g s[i] + i h s[i-1] per direction.
+template <int LT, class R>
+__device__ __forceinline__ void add_moments(const R (&g)[3], R h, R pref, R* E) {
+  R s[3][LT + 1];
 #pragma unroll
   for (int c = 0; c < 3; ++c) {
-    // G - A = (a2 (B - A) + a3 (C - A)) / z3, G - B = (-a1 (B - A) + a3 (C - B)) / z3
-    const float ba = (float)(B[c] - A[c]), ca = (float)(Cc[c] - A[c]), cb = (float)(Cc[c] - B[c]);
-    const float ga = ((float)a2 * ba + (float)a3 * ca) * iz3;
-    const float gb = (-(float)a1 * ba + (float)a3 * cb) * iz3;
-    os1d<L1, L2, float>(ga, gb, 0.5f * iz3, s[c]);
+    s[c][0] = R(1);
+#pragma unroll
+    for (int i = 1; i <= LT; ++i) {
+      R v = g[c] * s[c][i - 1];
+      if (i > 1) v += R(i - 1) * h * s[c][i - 2];
+      s[c][i] = v;
+    }
   }
-  const float r = 3.14159265358979f * iz3;
-  const float pref = (float)(w * expAB) * r * sqrtf(r) * expf(-(float)rho);
 #pragma unroll
-  for (int a = 0; a < N1; ++a)
+  for (int x = 0; x <= LT; ++x) {
+    const R px = x ? pref * s[0][x] : pref;
 #pragma unroll
-    for (int b = 0; b < N2; ++b)
-      cart[a * N2 + b] += pref * s[0][cex(a)][cex(b)] * s[1][cey(a)][cey(b)] * s[2][cez(a)][cez(b)];
+    for (int y = 0; y <= LT - x; ++y) {
+      const R pxy = y ? px * s[1][y] : px;
+#pragma unroll
+      for (int z = 0; z <= LT - x - y; ++z) {
+        if (z) E[midx(LT, x, y, z)] += pxy * s[2][z];
+        else E[midx(LT, x, y, z)] += pxy;
+      }
+    }
+  }
+}
+
+// cart(a, b) = sum_e coef(e) E(e), one direction after the other (z, y, x):
+// (y + PA)^a (y + PB)^b = sum_i c[a][b][i] y^i.
+template <int L1, int L2>
+__device__ __forceinline__ void moments_to_cart(const double* E, const double (&PA)[3], const double (&PB)[3],
+                                                double* cart) {
+  constexpr int LT = L1 + L2, N2 = ncart(L2);
+  double c[3][L1 + 1][L2 + 1][LT + 1];
+#pragma unroll
+  for (int d = 0; d < 3; ++d)
+#pragma unroll
+    for (int a = 0; a <= L1; ++a)
+#pragma unroll
+      for (int b = 0; b <= L2; ++b)
+#pragma unroll
+        for (int i = 0; i <= a + b; ++i) {
+          double v = 0.0;
+          if (a == 0 && b == 0) v = 1.0;
+          else if (a > 0) v = (i > 0 ? c[d][a - 1][b][i - 1] : 0.0) + (i < a + b ? PA[d] * c[d][a - 1][b][i] : 0.0);
+          else v = (i > 0 ? c[d][a][b - 1][i - 1] : 0.0) + (i < a + b ? PB[d] * c[d][a][b - 1][i] : 0.0);
+          c[d][a][b][i] = v;
+        }
+#pragma unroll
+  for (int az = 0; az <= L1; ++az)
+#pragma unroll
+    for (int bz = 0; bz <= L2; ++bz) {
+      const int rz = LT - az - bz;
+      double F[LT + 1][LT + 1];
+#pragma unroll
+      for (int x = 0; x <= rz; ++x)
+#pragma unroll
+        for (int y = 0; y <= rz - x; ++y) {
+          double v = E[midx(LT, x, y, az + bz)];
+#pragma unroll
+          for (int k = 0; k < az + bz; ++k) v += c[2][az][bz][k] * E[midx(LT, x, y, k)];
+          F[x][y] = v;
+        }
+#pragma unroll
+      for (int ay = 0; ay <= L1 - az; ++ay)
+#pragma unroll
+        for (int by = 0; by <= L2 - bz; ++by) {
+          const int ry = rz - ay - by;
+          double G[LT + 1];
+#pragma unroll
+          for (int x = 0; x <= ry; ++x) {
+            double v = F[x][ay + by];
+#pragma unroll
+            for (int k = 0; k < ay + by; ++k) v += c[1][ay][by][k] * F[x][k];
+            G[x] = v;
+          }
+#pragma unroll
+          for (int ax = 0; ax <= L1 - az - ay; ++ax)
+#pragma unroll
+            for (int bx = 0; bx <= L2 - bz - by; ++bx) {
+              double v = G[ax + bx];
+#pragma unroll
+              for (int k = 0; k < ax + bx; ++k) v += c[0][ax][bx][k] * G[k];
+              cart[cidx(ax, ay, az) * N2 + cidx(bx, by, bz)] = v;
+            }
+        }
+    }
+}
+
+// Far-shell split of the electronic potential.  With rho = z a3 / z3 |P - C|^2
+// an image enters with the suppression exp(-rho); images past kFarRho
+// (exp(-22) = 2.8e-10) may run in FP32 (GB300's FP32 rate is 64x its FP64
+// rate).  Their FP32 rounding, 6e-8 of a term that the suppression and the
+// recurrence's polynomial in the image distance (up to 25^4 for d-d at the
+// cut-off radius) keep below ~3e-6 of the block scale, stays near 2e-13 of
+// it.
+constexpr double kFarRho = 22.0;
+
+// a - b of two numbers held as unevaluated FP32 pairs (Knuth's two-sum).
+__device__ __forceinline__ void pair_sub(float ah, float al, float bh, float bl, float& h, float& l) {
+  const float s = __fsub_rn(ah, bh), v = __fsub_rn(s, ah);
+  const float e = __fadd_rn(__fsub_rn(__fsub_rn(ah, __fsub_rn(s, v)), __fadd_rn(bh, v)), __fsub_rn(al, bl));
+  h = __fadd_rn(s, e);
+  l = __fsub_rn(e, __fsub_rn(h, s));
+}
+__device__ __forceinline__ void two_sum(float a, float b, float& s, float& e) {
+  s = __fadd_rn(a, b);
+  const float v = __fsub_rn(s, a);
+  e = __fadd_rn(__fsub_rn(a, __fsub_rn(s, v)), __fsub_rn(b, v));
 }
 
 // ---------------------------------------------------------------------------
@@ -512,6 +601,46 @@ __device__ __forceinline__ void add_nuclear(double a1, double a2, double a3, con
       }
       cart[a * N2 + b] += acc;
     }
+}
+
+// Moments about P of one image of the nuclear operator: the vertical
+// recurrence of add_nuclear on the centre P (y^e in place of (r - A)^e),
+//   V(e+1_d, m) = GP_d V(e, m) - GC_d V(e, m+1)
+//                 + N_d(e) / (2 z3) [V(e-1_d, m) - V(e-1_d, m+1)],
+// added to E for m = 0.  GP = G - P, GC = G - C, pre the prefactor of
+// V(0, m) = pre F_m.  Only one order m is live at a time (from LT down).
+template <int LT>
+__device__ __forceinline__ void add_nuclear_moments(const double (&GP)[3], const double (&GC)[3], double inv2z3,
+                                                    double pre, const double (&F)[LT + 1], double* E) {
+  constexpr int NM = nmom(LT);
+  double V[NM];          // V(e, m + 1) on entry of the pass for m, |e| <= LT - m - 1
+  V[0] = pre * F[LT];
+#pragma unroll
+  for (int m = LT - 1; m >= 0; --m) {
+    double W[NM];
+    W[0] = pre * F[m];
+#pragma unroll
+    for (int s = 1; s <= LT - m; ++s)
+#pragma unroll
+      for (int x = s; x >= 0; --x)
+#pragma unroll
+        for (int y = s - x; y >= 0; --y) {
+          const int zz = s - x - y;
+          const int d = x > 0 ? 0 : (y > 0 ? 1 : 2);
+          const int px = x - (d == 0), py = y - (d == 1), pz = zz - (d == 2);
+          const int pe = d == 0 ? px : d == 1 ? py : pz;
+          double v = GP[d] * W[midx(LT, px, py, pz)] - GC[d] * V[midx(LT, px, py, pz)];
+          if (pe > 0) {
+            const int q = midx(LT, px - (d == 0), py - (d == 1), pz - (d == 2));
+            v += pe * inv2z3 * (W[q] - V[q]);
+          }
+          W[midx(LT, x, y, zz)] = v;
+        }
+#pragma unroll
+    for (int q = 0; q < NM; ++q) V[q] = W[q];
+  }
+#pragma unroll
+  for (int q = 0; q < NM; ++q) E[q] += V[q];
 }
 
 }  // namespace olc

@@ -115,6 +115,92 @@ int upload(olc_context* ctx, T** dst, const std::vector<T>& src) {
                     "upload");
 }
 
+// Images of the potential sites around every atom (SysView::img_*).  For an
+// alpha pair (a1 on A, a2 on B') at the fraction f = |A - B'|^2 / alphaDist of
+// its own cut-off the pair centre P lies at |A - P|^2 = f T a2 / (a1 (a1 + a2))
+// and its third-centre radius is R^2 = (1 - f) T (1 / a3 + 1 / (a1 + a2))
+// (gaussRelations.f90:138-278), so |A - P| + R <= sqrt(T (1 / a1 + 1 / a3)):
+// that radius, at the smallest exponents, bounds the list.
+// Within a group the images are ordered by distance shells of rad / kShells
+// (a counting sort; the kernels stop at the first shell past their reach).
+constexpr int kShells = 64;
+
+struct Images {
+  std::vector<int32_t> start;
+  std::vector<double4_16a> d;
+  std::vector<float4> hi, lo;
+};
+
+void make_images(const Lattice& lat, const olc_context* ctx, const std::vector<int32_t>& siteType,
+                 const std::vector<double>& sitePos, const double* potPos, const std::vector<double>& elemAlpha,
+                 const std::vector<double>& elemPot, const std::vector<double>& elemNuc, double T, Images& im) {
+  const int ns = (int)siteType.size();
+  double plane[3];            // spacing of the lattice planes, inverted
+  for (int l = 0; l < 3; ++l)
+    plane[l] = std::sqrt(lat.inv[l][0] * lat.inv[l][0] + lat.inv[l][1] * lat.inv[l][1] + lat.inv[l][2] * lat.inv[l][2]);
+  im.start.push_back(0);
+  std::vector<double4_16a> found;     // w = |C' - A|^2
+  for (int i = 0; i < ns; ++i) {
+    const DevType& t1 = ctx->htypes[siteType[i]];
+    const double a1 = elemAlpha[(size_t)t1.element * OLC_MAX_ALPHAS];
+    for (const DevPotType& pt : ctx->hpots) {
+      double a3 = elemPot[(size_t)pt.element * OLC_MAX_POT_ALPHAS];
+      for (int j = 1; j < pt.num_alphas; ++j)
+        a3 = std::min(a3, elemPot[(size_t)pt.element * OLC_MAX_POT_ALPHAS + j]);
+      if (pt.nuc_charge >= 1.0e-8) a3 = std::min(a3, elemNuc[pt.element]);
+      // an exponent of 0 (a bare charge, a type with more terms than its
+      // element's table) has no radius: every image of the cell list's extent
+      double rad = std::sqrt(T * (1.0 / a1 + 1.0 / a3)) * (1.0 + 1e-6);
+      if (!(a3 > 0.0) || !(rad < 1e6)) rad = std::sqrt(lat.cells.back());
+      const double rad2 = rad * rad;
+      found.clear();
+      for (int m = 0; m < pt.multiplicity; ++m) {
+        double v[3];
+        int lo[3], hi[3];
+        for (int c = 0; c < 3; ++c) v[c] = potPos[3 * (pt.first_site + m) + c] - sitePos[3 * i + c];
+        for (int l = 0; l < 3; ++l) {
+          // lattice planes of direction l within the radius (the margin
+          // covers the rounding of f)
+          const double f = v[0] * lat.inv[l][0] + v[1] * lat.inv[l][1] + v[2] * lat.inv[l][2];
+          const double w = rad * plane[l] + 1e-6;
+          lo[l] = (int)std::ceil(-f - w);
+          hi[l] = (int)std::floor(-f + w);
+        }
+        for (int n0 = lo[0]; n0 <= hi[0]; ++n0)
+          for (int n1 = lo[1]; n1 <= hi[1]; ++n1) {
+            double y[3];
+            for (int c = 0; c < 3; ++c) y[c] = lat.rv[0][c] * n0 + lat.rv[1][c] * n1;
+            for (int n2 = lo[2]; n2 <= hi[2]; ++n2) {
+              double x[3], d2 = 0.0;
+              for (int c = 0; c < 3; ++c) {
+                x[c] = v[c] + (y[c] + lat.rv[2][c] * n2);
+                d2 += x[c] * x[c];
+              }
+              if (d2 <= rad2) found.push_back(make_double4_16a(x[0], x[1], x[2], d2));
+            }
+          }
+      }
+      auto shell = [&](double d2) { return std::min(kShells - 1, (int)(kShells * std::sqrt(d2) / rad)); };
+      int32_t at[kShells + 1] = {};
+      for (const auto& x : found) ++at[shell(x.w) + 1];
+      for (int q = 0; q < kShells; ++q) at[q + 1] += at[q];
+      const size_t base = im.d.size();
+      im.d.resize(base + found.size());
+      im.hi.resize(base + found.size());
+      im.lo.resize(base + found.size());
+      for (const auto& x : found) {
+        const int q = shell(x.w);
+        const size_t o = base + at[q]++;
+        const float4 h = make_float4((float)x.x, (float)x.y, (float)x.z, (float)(0.999999 * rad / kShells * q));
+        im.d[o] = x;
+        im.hi[o] = h;
+        im.lo[o] = make_float4((float)(x.x - h.x), (float)(x.y - h.y), (float)(x.z - h.z), 0.f);
+      }
+      im.start.push_back((int32_t)im.d.size());
+    }
+  }
+}
+
 int lmax_of_alpha(const olc_atom_type_t& t, int a /*0-based*/) {
   int j = a + 1;
   if (j <= t.num_orb_alphas[3]) return 3;
@@ -332,21 +418,35 @@ int build_system(olc_context* ctx, const olc_system_t* s) {
   const int ntasks = (int)ctx->htasks.size();
 
   // ---- alpha-pair items grouped by (l1, l2) class -------------------------
+  // The pairs of two types, the most diffuse first: the third-centre radius
+  // falls with a1 + a2, so neighbouring threads of the primitive kernels sum
+  // about the same number of images.
+  struct AlphaPair {
+    double dist, sum;
+    int cls;
+    int32_t ab;
+  };
+  std::vector<std::vector<AlphaPair>> typePairs((size_t)s->num_atom_types * s->num_atom_types);
+  for (int x = 0; x < s->num_atom_types; ++x)
+    for (int y = 0; y < s->num_atom_types; ++y) {
+      const DevType &t1 = ctx->htypes[x], &t2 = ctx->htypes[y];
+      auto& tp = typePairs[(size_t)x * s->num_atom_types + y];
+      for (int a1 = 0; a1 < t1.nalpha; ++a1)
+        for (int a2 = 0; a2 < t2.nalpha; ++a2)
+          tp.push_back({alphaDist(a1, a2, t1.element, t2.element), t1.alphas[a1] + t2.alphas[a2],
+                        t1.lmax_alpha[a1] * (kMaxL + 1) + t2.lmax_alpha[a2], a1 | (a2 << 8)});
+      std::stable_sort(tp.begin(), tp.end(), [](const AlphaPair& p, const AlphaPair& q) { return p.sum < q.sum; });
+    }
   std::vector<int32_t> itTask[kNumClasses], itAB[kNumClasses], itStart[kNumClasses];
   for (int c = 0; c < kNumClasses; ++c) itStart[c].assign(ntasks + 1, 0);
   for (int q = 0; q < ntasks; ++q) {
     const DevTask& tk = ctx->htasks[q];
     const DevPair& p = ctx->hpairs[tk.pair];
-    const DevType& t1 = ctx->htypes[siteType[p.i]];
-    const DevType& t2 = ctx->htypes[siteType[p.j]];
     for (int c = 0; c < kNumClasses; ++c) itStart[c][q] = (int32_t)itTask[c].size();
-    for (int a1 = 0; a1 < t1.nalpha; ++a1) {
-      for (int a2 = 0; a2 < t2.nalpha; ++a2) {
-        if (alphaDist(a1, a2, t1.element, t2.element) < tk.sep) break;
-        int cls = t1.lmax_alpha[a1] * (kMaxL + 1) + t2.lmax_alpha[a2];
-        itTask[cls].push_back(q);
-        itAB[cls].push_back(a1 | (a2 << 8));
-      }
+    for (const AlphaPair& e : typePairs[(size_t)siteType[p.i] * s->num_atom_types + siteType[p.j]]) {
+      if (e.dist < tk.sep) continue;
+      itTask[e.cls].push_back(q);
+      itAB[e.cls].push_back(e.ab);
     }
   }
   for (int c = 0; c < kNumClasses; ++c) itStart[c][ntasks] = (int32_t)itTask[c].size();
@@ -398,6 +498,20 @@ int build_system(olc_context* ctx, const olc_system_t* s) {
   if ((st = upload(ctx, &dst, potType))) return st;
   v.pot_site_type = dst;
   v.num_pot_sites = s->num_pot_sites;
+  {
+    Images im;
+    make_images(lat, ctx, siteType, sitePos, s->pot_site_pos, elemAlpha, elemPot, elemNuc, T, im);
+    double4_16a* d4;
+    float4* f4;
+    if ((st = upload(ctx, &dst, im.start))) return st;
+    v.img_start = dst;
+    if ((st = upload(ctx, &d4, im.d))) return st;
+    v.img_d = d4;
+    if ((st = upload(ctx, &f4, im.hi))) return st;
+    v.img_hi = f4;
+    if ((st = upload(ctx, &f4, im.lo))) return st;
+    v.img_lo = f4;
+  }
   if ((st = upload(ctx, &dd, elemAlpha))) return st;
   v.elem_alpha = dd;
   if ((st = upload(ctx, &dd, elemNuc))) return st;
