@@ -110,11 +110,6 @@ int olc_create(const olc_system_t* sys, void* stream, olc_context_t** out) {
   olc_context* ctx = new olc_context();
   ctx->device = dev;
   ctx->stream = static_cast<cudaStream_t>(stream);
-  if (cusolverDnCreate(&ctx->solver) != CUSOLVER_STATUS_SUCCESS) {
-    delete ctx;
-    return fail(OLC_ERR_CUDA, "cusolverDnCreate failed");
-  }
-  cusolverDnSetStream(ctx->solver, ctx->stream);
   {
     cudaMemPoolProps props = {};
     props.allocType = cudaMemAllocationTypePinned;
@@ -183,7 +178,7 @@ int olc_get_dims(const olc_context_t* ctx, olc_dims_t* dims) {
 int olc_set_stream(olc_context_t* ctx, void* stream) {
   if (!ctx) return fail(OLC_ERR_ARG, "olc_set_stream: null context");
   ctx->stream = static_cast<cudaStream_t>(stream);
-  cusolverDnSetStream(ctx->solver, ctx->stream);
+  if (ctx->solver) cusolverDnSetStream(ctx->solver, ctx->stream);
   return OLC_OK;
 }
 
