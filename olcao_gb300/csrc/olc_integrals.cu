@@ -7,9 +7,9 @@
 //   and the third-centre sums of nuclearPE / electronicPE (integrals.F90:
 //   2275-2598) -- producing the harmonic block sh(lm1, lm2) of each item in
 //   a scratch buffer.
-// Stage 2 (contraction, one warp per (pair, cell) task): the accumulation
-//   into pairXBasisFn2 and multWithBasisFn1 (integrals.F90:402-410,
-//   intgSaving.F90:56-89) as one sum over the task's items,
+// Stage 2 (contraction, one CTA per (pair, cell) task and column block): the
+//   accumulation into pairXBasisFn2 and multWithBasisFn1 (integrals.F90:
+//   402-410, intgSaving.F90:56-89), in the same two steps,
 //   block(m1,m2) = sum c1(a1,m1) c2(a2,m2) sh(lm(m1), lm(m2)).
 // Stage 3 (Bloch sum + scatter, one CTA per (pair, k range)):
 //   applyPhaseFactors, kPointLatticeOriginShift and saveCurrentPair
@@ -100,46 +100,92 @@ int run_primitives(olc_context* ctx, int op, int term, const double* coeffs, int
 }
 
 // ---------------------------------------------------------------------------
-// stage 2: contraction with the basis coefficients, one warp per task
+// stage 2: contraction with the basis coefficients
 // ---------------------------------------------------------------------------
 struct ContractArgs {
   const int32_t* ab[kNumClasses];
   const int32_t* start[kNumClasses];
   const double* sh[kNumClasses];
-  int ntasks;
   int ms;                   // block stride (max states)
+  int rows;                 // rows of the half-contracted table (exponents x harmonics)
   double* block;            // [task][m2*ms + m1]
 };
 
-__global__ void __launch_bounds__(256) contract_kernel(SysView v, ContractArgs a) {
-  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (warp >= a.ntasks) return;
-  const DevTask tk = v.tasks[warp];
-  const DevPair p = v.pairs[tk.pair];
+// One CTA per (task, kContractCols states of the second atom).  The FP64 pipe
+// bounds the contraction, so it runs in two steps, as pairXBasisFn2 and
+// multWithBasisFn1 do: T(a1, lm1; m2) = sum_a2 c2(a2, m2) sh(a1, a2; lm1, lm2)
+// in shared memory, then block(m1, m2) = sum_a1 c1(a1, m1) T(a1, lm(m1); m2)
+// -- about 9 n_a^2 M2 + n_a M1 M2 multiply-adds where one sum per element over
+// all alpha pairs costs 3 n_a^2 M1 M2 operations.  Per operator: two-atom cell
+// with f functions 1.32 -> 0.10 ms, 64-atom silicon cell 1.12 -> 0.7 ms, two-atom
+// silicon cell 0.57 -> 0.07 ms.
+constexpr int kContractCols = 8;
+constexpr int kContractThreads = 128;
+
+__global__ void __launch_bounds__(kContractThreads) contract_kernel(SysView v, ContractArgs a) {
+  __shared__ const double* item[OLC_MAX_ALPHAS * OLC_MAX_ALPHAS];   // sh block of (a1, a2), null: none
+  __shared__ double c2[kContractCols][OLC_MAX_ALPHAS];
+  __shared__ int used[OLC_MAX_ALPHAS], w2[OLC_MAX_ALPHAS];        // a2 range of each a1; harmonics of each a2
+  __shared__ int nrow;
+  extern __shared__ double half[];                       // [column][a1 * ns1 + lm1]
+  const int task = blockIdx.x, tid = threadIdx.x;
+  const DevPair& p = v.pairs[v.tasks[task].pair];
   const DevType& t1 = v.types[v.site_type[p.i]];
   const DevType& t2 = v.types[v.site_type[p.j]];
-  const int M1 = t1.nstates, M2 = t2.nstates;
-  double* out = a.block + (size_t)warp * a.ms * a.ms;
-  for (int e = lane; e < M1 * M2; e += 32) {
-    const int m1 = e % M1, m2 = e / M1;
-    const int lm1 = t1.lm_index[m1] - 1, lm2 = t2.lm_index[m2] - 1;
-    double acc = 0.0;
+  const int M1 = t1.nstates, M2 = t2.nstates, c0 = blockIdx.y * kContractCols;
+  if (c0 >= M2) return;
+  const int mc = min(kContractCols, M2 - c0);
+  const int n1 = t1.nalpha, n2 = t2.nalpha;
+  const int ns1 = (t1.lmax_alpha[0] + 1) * (t1.lmax_alpha[0] + 1);
+  for (int e = tid; e < n1 * n2; e += kContractThreads) item[e] = nullptr;
+  for (int e = tid; e < n2 * mc; e += kContractThreads)
+    c2[e / n2][e % n2] = t2.basis[(e % n2) * OLC_MAX_STATES + c0 + e / n2];
+  if (tid < OLC_MAX_ALPHAS) {
+    used[tid] = 0;
+    const int l2 = tid < n2 ? t2.lmax_alpha[tid] : -1;
+    w2[tid] = (l2 + 1) * (l2 + 1);
+  }
+  if (tid == 0) nrow = 0;
+  __syncthreads();
 #pragma unroll
-    for (int cls = 0; cls < kNumClasses; ++cls) {
-      const int l1 = cls / (kMaxL + 1), l2 = cls % (kMaxL + 1);
-      const int ns1 = (l1 + 1) * (l1 + 1), ns2 = (l2 + 1) * (l2 + 1);
-      if (lm1 >= ns1 || lm2 >= ns2) continue;
-      const int b = a.start[cls][warp], en = a.start[cls][warp + 1];
-      const double* sh = a.sh[cls];
-      for (int q = b; q < en; ++q) {
-        const int ab = a.ab[cls][q];
-        const int a1 = ab & 255, a2 = ab >> 8;
-        acc += t1.basis[a1 * OLC_MAX_STATES + m1] * t2.basis[a2 * OLC_MAX_STATES + m2] *
-               sh[(size_t)q * ns1 * ns2 + lm2 * ns1 + lm1];
+  for (int cls = 0; cls < kNumClasses; ++cls) {
+    const int wi = (cls / (kMaxL + 1) + 1) * (cls / (kMaxL + 1) + 1), wj = (cls % (kMaxL + 1) + 1) * (cls % (kMaxL + 1) + 1);
+    const int b = a.start[cls][task], en = a.start[cls][task + 1];
+    for (int q = b + tid; q < en; q += kContractThreads) {
+      const int ab = a.ab[cls][q], a1 = ab & 255, a2 = ab >> 8;
+      item[a1 * n2 + a2] = a.sh[cls] + (size_t)q * (wi * wj);
+      atomicMax(&used[a1], a2 + 1);
+      atomicMax(&nrow, a1 + 1);
+    }
+  }
+  __syncthreads();
+  const int rows = nrow * ns1;
+  for (int e = tid; e < rows * mc; e += kContractThreads) {
+    const int row = e % rows, c = e / rows;
+    const int a1 = row / ns1, lm1 = row % ns1;
+    const int l1 = t1.lmax_alpha[a1], w1 = (l1 + 1) * (l1 + 1);
+    double acc = 0.0;
+    if (lm1 < w1) {
+      const int lm2 = t2.lm_index[c0 + c] - 1, off = lm2 * w1 + lm1, na = used[a1];
+      const double* const* it = item + a1 * n2;
+      // the loads of six exponents in flight together
+#pragma unroll 6
+      for (int a2 = 0; a2 < na; ++a2) {
+        const double* s = it[a2];
+        if (s && lm2 < w2[a2]) acc = fma(c2[c][a2], s[off], acc);
       }
     }
-    out[m2 * a.ms + m1] = acc;
+    half[c * a.rows + row] = acc;
+  }
+  __syncthreads();
+  double* out = a.block + (size_t)task * a.ms * a.ms;
+  for (int e = tid; e < M1 * mc; e += kContractThreads) {
+    const int m1 = e % M1, c = e / M1, lm1 = t1.lm_index[m1] - 1;
+    double acc = 0.0;
+#pragma unroll 4
+    for (int a1 = 0; a1 < nrow; ++a1)
+      acc = fma(t1.basis[a1 * OLC_MAX_STATES + m1], half[c * a.rows + a1 * ns1 + lm1], acc);
+    out[(c0 + c) * a.ms + m1] = acc;
   }
 }
 
@@ -249,12 +295,18 @@ int run_contract_bloch(olc_context* ctx, double* vv, double* cv, double* cc) {
     ca.start[c] = ctx->items.task_start[c];
     ca.sh[c] = ctx->d_sh + ctx->items.sh_offset[c];
   }
-  ca.ntasks = ntasks;
   ca.ms = ctx->max_states;
   ca.block = ctx->d_block;
+  ca.rows = 0;
+  for (const DevType& t : ctx->htypes)
+    ca.rows = std::max(ca.rows, t.nalpha * (t.lmax_alpha[0] + 1) * (t.lmax_alpha[0] + 1));
+  const size_t csmem = sizeof(double) * kContractCols * (size_t)ca.rows;
+  if ((st = cuda_check(cudaFuncSetAttribute(contract_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)csmem),
+                       "contract smem"))) return st;
   {
     StageScope scope(ctx, OLC_STAGE_CONTRACT);
-    contract_kernel<<<(ntasks + 7) / 8, 256, 0, ctx->stream>>>(v, ca);
+    const dim3 cgrid((unsigned)ntasks, (unsigned)((ctx->max_states + kContractCols - 1) / kContractCols));
+    contract_kernel<<<cgrid, kContractThreads, csmem, ctx->stream>>>(v, ca);
   }
   if ((st = cuda_check(cudaGetLastError(), "contract_kernel"))) return st;
   BlochArgs ba;
