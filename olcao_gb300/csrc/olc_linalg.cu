@@ -21,7 +21,7 @@
 
 namespace olc {
 
-int solve_small_batched(olc_context* ctx, const double* h_full, const double* s_full, int n,
+int solve_small_batched(olc_context* ctx, const double* h_full, double* s_full, int n,
                         int num_states, double* eigenvalues, double* vectors, int32_t* info_host,
                         bool s_is_factored);
 int small_solver_max_n();

@@ -15,7 +15,7 @@
 
 namespace olc {
 
-int launch_small_hegv_raw(cudaStream_t stream, const double* h_full, const double* s_full, int n,
+int launch_small_hegv_raw(cudaStream_t stream, const double* h_full, double* s_full, int n,
                           int nk, int num_states, double* eigenvalues, double* vectors,
                           int32_t* info_dev);
 int small_solver_capacity_n();
