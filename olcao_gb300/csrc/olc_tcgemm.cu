@@ -635,6 +635,37 @@ __global__ void slice_b_kernel(const T* __restrict__ src, long long sstride, int
   }
 }
 
+// Right operand planes of B = src^H (src n x k, column-major), FP32 pieces: the
+// rows of slice_b_kernel, 32 x 32 tiles through shared memory.
+__global__ void __launch_bounds__(256) slice_bh_kernel(const float* __restrict__ src, long long sstride, int ld, int k,
+                                                       int n, int kp, __nv_bfloat16* __restrict__ out) {
+  __shared__ float2 tile[32][33];                         // [column of B][K index]
+  const int b = blockIdx.z, c0 = blockIdx.x * 32, r0 = blockIdx.y * 32;
+  const int tx = threadIdx.x, ty = threadIdx.y;
+  const float2* s = reinterpret_cast<const float2*>(src + (size_t)b * sstride);
+  for (int j = ty; j < 32; j += 8) {
+    const int c = c0 + tx, r = r0 + j;
+    tile[tx][j] = (c < n && r < k) ? s[(size_t)r * ld + c] : make_float2(0.f, 0.f);
+  }
+  __syncthreads();
+  const size_t Kp = 2 * (size_t)kp;
+  for (int j = ty; j < 32; j += 8) {
+    const int c = c0 + j, r = r0 + tx;
+    if (c >= n || r >= kp) continue;
+    float vr = tile[j][tx].x, vi = -tile[j][tx].y;
+    for (int pl = 0; pl < 3; ++pl) {
+      const __nv_bfloat16 pr = __float2bfloat16_rn(vr), pi = __float2bfloat16_rn(vi);
+      __nv_bfloat16* o = out + (((size_t)b * 3 + pl) * 2 * n + 2 * (size_t)c) * Kp;
+      o[r] = pr;
+      o[kp + r] = __float2bfloat16_rn(-__bfloat162float(pi));
+      o[Kp + r] = pi;
+      o[Kp + kp + r] = pr;
+      vr -= __bfloat162float(pr);
+      vi -= __bfloat162float(pi);
+    }
+  }
+}
+
 int grid_of(size_t n) { return (int)std::min<size_t>((n + 255) / 256, 152 * 16); }
 
 // C(r, c) = conj(C(c, r)) for r > c: the strict lower triangle of a
@@ -852,7 +883,7 @@ int zgemm_fixed(olc_context* ctx, int m, int n, int k, const TA* A, long long sA
 
 int cgemm_f32(olc_context* ctx, int m, int n, int k, const float* A, long long sA, int lda, bool conjA,
               const float* B, long long sB, int ldb, float alpha, float beta, float* C, long long sC, int ldc,
-              int nb, int stage, bool lower, int tri) {
+              int nb, int stage, bool lower, int tri, bool conjB) {
   cudaStream_t st = ctx->stream;
   const int kp = (k + 31) & ~31;
   const size_t Kp = 2 * (size_t)kp;
@@ -876,8 +907,11 @@ int cgemm_f32(olc_context* ctx, int m, int n, int k, const float* A, long long s
     const float* Bb = B + (size_t)b0 * sB;
     slice_a_kernel<float><<<dim3((m + 31) / 32, (kp + 31) / 32, cb), dim3(32, 8), 0, st>>>(
         Ab, sA, lda, conjA, m, k, kp, nullptr, 3, 0, false, wa);
-    slice_b_kernel<float><<<grid_of((size_t)kp * n * cb), 256, 0, st>>>(Bb, sB, ldb, k, n, kp, nullptr, 3, 0, false,
-                                                                        cb, wb);
+    if (conjB)
+      slice_bh_kernel<<<dim3((n + 31) / 32, (kp + 31) / 32, cb), dim3(32, 8), 0, st>>>(Bb, sB, ldb, k, n, kp, wb);
+    else
+      slice_b_kernel<float><<<grid_of((size_t)kp * n * cb), 256, 0, st>>>(Bb, sB, ldb, k, n, kp, nullptr, 3, 0, false,
+                                                                          cb, wb);
     scope.add_launches(2);
     TcParams p{};
     p.m = m;

@@ -60,9 +60,11 @@ constexpr int kTriAUpper = 1, kTriALower = 2, kTriBUpper = 4;
 // three BF16 pieces per FP32 operand (six piece pairs).  lower: only the
 // output tiles that reach the lower triangle (row >= column) are formed; the
 // rest of C keeps its values.  tri: kTri* flags of triangular operands.
+// conjB: the product takes the conjugate transpose of the array at B (n x k,
+// leading dimension ldb).
 int cgemm_f32(olc_context* ctx, int m, int n, int k, const float* A, long long sA, int lda, bool conjA,
               const float* B, long long sB, int ldb, float alpha, float beta, float* C, long long sC, int ldc,
-              int nb, int stage, bool lower = false, int tri = 0);
+              int nb, int stage, bool lower = false, int tri = 0, bool conjB = false);
 
 // Digits and kept pairs of a fixed-point product (see olc_tcgemm.cu).
 void fixed_plan(int bits_a, int bits_b, int prec, int* na, int* nbd, int* T);
