@@ -1,8 +1,8 @@
 // Blackwell tensor-core GEMM for the complex products of the mixed solver:
 // tcgen05.mma issued by one thread, BF16 operands staged by TMA
-// (cp.async.bulk.tensor) into 128-byte-swizzled shared memory through a
-// four-stage mbarrier pipeline, FP32 accumulators in tensor memory (TMEM)
-// drained by eight epilogue warps with tcgen05.ld.
+// (cp.async.bulk.tensor) into 128-byte-swizzled shared memory through rings
+// of plane slots guarded by mbarriers, FP32 accumulators in tensor memory (TMEM)
+// drained by the epilogue warps with tcgen05.ld.
 //
 // Complex products as one real GEMM.  For C = op(A) B (A: m x k, B: k x n
 // complex) the kernel computes the real product D = A' B'^T with
@@ -14,23 +14,26 @@
 // are K-major (K contiguous), the layout tcgen05 reads without transposition.
 //
 // Operands are "planes" of BF16 values: digit planes of a fixed-point split
-// or the three BF16 pieces of an FP32 number.  A launch runs a list of
-// segments (plane of A, plane of B, K-block range):
+// or the three BF16 pieces of an FP32 number.  Within one K-step (one or two
+// K-blocks, 64 of K' each) a launch runs a list of plane pairs; every plane's
+// tile is staged once per K-block, in a slot of its own, and stays until the
+// last pair that uses it.  The pairs form groups that share an accumulator;
+// the epilogue drains a group's sums from one TMEM accumulator while the
+// tensor cores fill the next.
 //
 //  * fixed mode (FP64-accurate products): every row of op(A) and column of B
-//    is scaled by a power of two and cut into signed 8-bit digits
-//    (|d| <= 255: BF16 holds every integer up to 256 exactly).  One segment is
-//    one digit pair (s, t) over at most 256 of K', so that its FP32 sum of at
-//    most 256 * 255^2 < 2^24
-//    is an exact integer.  Segments alternate between two TMEM accumulators;
-//    the epilogue drains each one (tcgen05.ld, exact float -> int) into
-//    64-bit fixed point, acc += g << shift(s + t), while the tensor cores fill
-//    the other.  Digit pairs whose weight is below the kept precision are not
-//    issued.  The result is acc scaled by 2^(e_row + f_col + base): FP64
-//    complex, no intermediate in global memory.
+//    is scaled by a power of two and cut into signed 8-bit digits, balanced
+//    (|d| <= 128, the leading digit up to 256; BF16 holds every integer up to
+//    256 exactly).  A group is the digit pairs (s, t) of one weight s + t; its
+//    FP32 sum over the K-step, at most 64 (2 2^15 + 5 2^14) or 128 (2 2^15 + 2^14),
+//    is below 2^24, an exact integer, drained (exact float -> int) into 64-bit fixed point,
+//    acc += g << shift(s + t).  Digit pairs whose weight is below the kept
+//    precision are not issued.  The result is acc scaled by
+//    2^(e_row + f_col + base): FP64 complex, no intermediate in global memory.
 //  * f32 mode (FP32-accurate products): x = x0 + x1 + x2 (three BF16 pieces
-//    of an FP32 value, 24 bits); the six pairs with weight >= 2^-16
-//    accumulate in one FP32 TMEM accumulator; C = alpha D + beta C.
+//    of an FP32 value, 24 bits); the six pairs with weight >= 2^-16 of one
+//    K-block (384 products) accumulate in an FP32 TMEM accumulator, which is
+//    drained into register sums; C = alpha D + beta C.
 //
 // GPU safety: every mbarrier wait is bounded by wall time (%globaltimer);
 // on expiry the thread records an error code, the other roles see it and
@@ -55,19 +58,18 @@ namespace {
 
 constexpr int BM = 128;            // rows per tile (TMEM lanes)
 constexpr int BK = 64;             // K per stage: 64 BF16 = one 128-byte swizzle row
-constexpr int STAGES = 4;
-constexpr int NUM_EPI_WARPS = 8;
-constexpr int NUM_THREADS = (NUM_EPI_WARPS + 2) * 32;
-constexpr int PRODUCER_WARP = NUM_EPI_WARPS;
-constexpr int MMA_WARP = NUM_EPI_WARPS + 1;
-// two accumulators of BN columns: 256 (fixed mode) or 512 (f32 mode)
+constexpr int MAX_SLOTS = 8;       // plane slots per operand
+// epilogue warps: the fixed mode's 64-bit sums want registers, the f32 mode's
+// drains want loads in flight
 template <int MODE>
-constexpr int tmem_cols() { return MODE == 0 ? 256 : 512; }
+constexpr int epi_warps() { return MODE == 0 ? 8 : 16; }
+template <int MODE>
+constexpr int num_threads() { return (epi_warps<MODE>() + 2) * 32; }
+// accumulators: four of 128 columns (fixed mode), two of 256 (f32 mode)
+template <int MODE>
+constexpr int num_acc() { return MODE == 0 ? 4 : 2; }
+constexpr int kTmemCols = 512;
 constexpr long long kWaitNs = 2000000000LL;   // 2 s per wait
-// fixed mode: K' per drained segment, the largest multiple of BK with
-// kChunkK (2^kBeta - 1)^2 < 2^24 (every FP32 partial sum an exact integer)
-constexpr int kChunkK = (int)((16777215LL / (((1LL << kBeta) - 1) * ((1LL << kBeta) - 1))) / BK * BK);
-static_assert(kChunkK >= BK, "digit width too large for exact FP32 segments");
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return (uint32_t)__cvta_generic_to_shared(p);
@@ -126,10 +128,14 @@ __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence:
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
 // Shared-memory matrix descriptor: K-major, 128-byte swizzle, 8-row atoms of
-// 1024 bytes (stride byte offset), descriptor version 1.
-__device__ __forceinline__ uint64_t sdesc(uint32_t saddr) {
-  return (uint64_t)((saddr >> 4) & 0x3FFF) | ((uint64_t)1 << 16) | ((uint64_t)(1024 >> 4) << 32) |
-         ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
+// 1024 bytes (stride byte offset), descriptor version 1.  lo: the address
+// field (bytes / 16) with kDescLo.
+constexpr uint32_t kDescLo = 1u << 16, kDescHi = (1024u >> 4) | (1u << 14) | (2u << 29);
+__device__ __forceinline__ uint64_t sdesc(uint32_t lo) { return ((uint64_t)kDescHi << 32) | lo; }
+__device__ __forceinline__ bool elect_one() {
+  uint32_t one;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(one));
+  return one != 0;
 }
 // Instruction descriptor of kind::f16: BF16 A and B, FP32 D, both K-major.
 __host__ __device__ constexpr uint32_t idesc_bf16(int M, int N) {
@@ -154,18 +160,6 @@ __device__ __forceinline__ void tmem_ld16(uint32_t ta, uint32_t (&r)[16]) {
         "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
       : "r"(ta));
 }
-// 32 consecutive 32-bit TMEM columns of this thread's lane
-__device__ __forceinline__ void tmem_ld32(uint32_t ta, uint32_t (&r)[32]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,"
-      "%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-        "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
-        "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]),
-        "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]),
-        "=r"(r[30]), "=r"(r[31])
-      : "r"(ta));
-}
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
 // Tile of a CTA: grouped raster (GM row tiles at a time) so that the CTAs in
@@ -180,43 +174,55 @@ __device__ __forceinline__ void tile_of(int t, int nmt, int nnt, int& mt, int& n
   nt = r / gsize;
 }
 
-struct SmemLayout {
-  static constexpr int a_bytes = BM * BK * 2;
-  template <int BN>
-  static constexpr int b_bytes() { return BN * BK * 2; }
-  template <int BN>
-  static constexpr int bars_offset() { return STAGES * (a_bytes + b_bytes<BN>()); }
-  template <int BN>
-  static constexpr int total() { return bars_offset<BN>() + 256 + 1024; }   // barriers + alignment slack
-};
+constexpr int kTileBytesA = BM * BK * 2;
+template <int MODE>
+constexpr int tile_bytes_b() { return (MODE == 0 ? 128 : 256) * BK * 2; }
+// planes' slots, barriers, alignment slack
+inline int smem_total(int mode, int slots_a, int slots_b) {
+  return slots_a * kTileBytesA + slots_b * (mode == 0 ? tile_bytes_b<0>() : tile_bytes_b<1>()) + 512 + 1024;
+}
 
 }  // namespace
 
 // ---------------------------------------------------------------------------
 // the kernel
 // ---------------------------------------------------------------------------
-// MODE 0 (fixed): BN = 128, two accumulators of 128 columns, int64 drains,
+// What bounds it: in the fixed mode the drains (a 128 x 128 accumulator through
+// tcgen05.ld, exact conversion and 64-bit multiply-adds) and the issue of the
+// MMAs, 79 clocks each at N = 128, run about level; in the f32 mode the copies'
+// latency at the K-steps' ends.  Measured: FP64-accurate product of order 1248
+// 1025 -> 850 us, FP32-accurate 78 -> 83 us (one partial wave), 64 products of
+// order 832 with 17 digit pairs 7.3 -> 6.1 ms each, the FP32-accurate products
+// of a pass over 8 matrices of order 2808 72 -> 55 ms.
+// MODE 0 (fixed): BN = 128, four accumulators of 128 columns, int64 drains,
 //   FP64 complex output.  Epilogue warp w owns TMEM lanes 32 (w % 4) .. +31
-//   and columns 64 (w / 4) .. +63 of the tile (32 complex columns).
-// MODE 1 (f32):   BN = 256, one accumulator, FP32 complex output with
-//   alpha, beta; warp w owns columns 128 (w / 4) .. +127 (64 complex).
+//   and columns 32 (w / 4) .. +31 of the tile (16 complex columns).
+// MODE 1 (f32):   BN = 256, two accumulators, FP32 complex output with
+//   alpha, beta; warp w owns columns 64 (w / 4) .. +63 (32 complex).
+
 template <int MODE>
-__global__ void __launch_bounds__(NUM_THREADS, 1)
+__global__ void __launch_bounds__(num_threads<MODE>(), 1)
     tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                    const __grid_constant__ TcParams p) {
   constexpr int BN = MODE == 0 ? 128 : 256;
+  constexpr int NACC = num_acc<MODE>();
   constexpr uint32_t IDESC = idesc_bf16(BM, BN);
+  constexpr int TB = tile_bytes_b<MODE>();
+  constexpr int PRODUCER_WARP = epi_warps<MODE>(), MMA_WARP = PRODUCER_WARP + 1;
+  constexpr int CW = 4 * BN / epi_warps<MODE>();      // columns of an epilogue warp
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   uint8_t* smem = smem_raw + (((raw + 1023u) & ~1023u) - raw);
   uint8_t* sA = smem;
-  uint8_t* sB = smem + STAGES * SmemLayout::a_bytes;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + SmemLayout::bars_offset<BN>());
-  uint64_t* full = bars;                 // [STAGES] TMA -> MMA
-  uint64_t* empty = bars + STAGES;       // [STAGES] MMA -> TMA
-  uint64_t* accfull = bars + 2 * STAGES; // [2] MMA -> epilogue
-  uint64_t* accempty = accfull + 2;      // [2] epilogue -> MMA
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(accempty + 2);
+  uint8_t* sB = smem + p.slots_a * kTileBytesA;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sB + p.slots_b * TB);
+  uint64_t* fullA = bars;                    // [slot] TMA -> MMA
+  uint64_t* emptyA = fullA + MAX_SLOTS;      // [slot] MMA -> TMA
+  uint64_t* fullB = emptyA + MAX_SLOTS;
+  uint64_t* emptyB = fullB + MAX_SLOTS;
+  uint64_t* accfull = emptyB + MAX_SLOTS;    // [NACC] MMA -> epilogue
+  uint64_t* accempty = accfull + 4;          // [NACC] epilogue -> MMA
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(accempty + 4);
   volatile int* cta_err = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -230,12 +236,9 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
   // lower part wanted: a tile whose complex columns all lie right of its last
   // row is wholly above the diagonal
   if (p.lower_only && (n0 >> 1) > m0 + BM - 1) return;
-  // segments: every pair over K chunks of chunk_blocks K-blocks
-  const int nchunk = (p.kblocks + p.chunk_blocks - 1) / p.chunk_blocks;
-  const int nseg = p.npairs * nchunk;
   // triangular operands (f32 mode): the complex K range [kmin, kmax) this
-  // tile needs; a K-block is issued when it meets that range in the real or
-  // the imaginary half of K' (every role skips the same blocks and segments)
+  // tile needs; a K-block is run when it meets that range in the real or the
+  // imaginary half of K' (every role skips the same blocks)
   int kmin = 0, kmax = p.kp;
   if (p.tri_a_upper) kmin = m0;
   if (p.tri_a_lower) kmax = min(kmax, m0 + BM);
@@ -246,22 +249,17 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
     const int lo = kb * BK, hi = lo + BK;
     return (lo < kmax && hi > kmin) || (lo < p.kp + kmax && hi > p.kp + kmin);
   };
-  auto seg_live = [&](int si) {
-    if (!tri) return true;
-    const int kb0 = (si % nchunk) * p.chunk_blocks, kb1 = min(p.kblocks, kb0 + p.chunk_blocks);
-    for (int kb = kb0; kb < kb1; ++kb)
-      if (kb_needed(kb)) return true;
-    return false;
-  };
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < STAGES; ++s) {
-      mbar_init(&full[s], 1);
-      mbar_init(&empty[s], 1);
+    for (int s = 0; s < MAX_SLOTS; ++s) {
+      mbar_init(&fullA[s], 1);
+      mbar_init(&emptyA[s], 1);
+      mbar_init(&fullB[s], 1);
+      mbar_init(&emptyB[s], 1);
     }
-    for (int s = 0; s < 2; ++s) {
+    for (int s = 0; s < NACC; ++s) {
       mbar_init(&accfull[s], 1);
-      mbar_init(&accempty[s], NUM_EPI_WARPS);
+      mbar_init(&accempty[s], epi_warps<MODE>());
     }
     *cta_err = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -269,7 +267,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
   }
   if (warp == MMA_WARP) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
-                 "r"(tmem_cols<MODE>()));
+                 "r"(kTmemCols));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
   tc_fence_before();
@@ -281,124 +279,152 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
     if (lane == 0) {
       asm volatile("prefetch.tensormap [%0];" ::"l"(&tmA) : "memory");
       asm volatile("prefetch.tensormap [%0];" ::"l"(&tmB) : "memory");
-      int stage = 0;
-      uint32_t phase = 0;
-      int issued = 0;   // stages filled (bounds the copies still in flight on the error path)
+      int sa = 0, sb = 0;               // next slots; their wrap-around parities
+      uint32_t pha = 0, phb = 0;
+      int na = 0, nb = 0;               // copies issued
+      const int span = p.kspan - 1;     // 0 or 1
       bool ok = true;
-      for (int si = 0; si < nseg && ok; ++si) {
-        const TcPair pr = p.pairs[si / nchunk];
-        const int kb0 = (si % nchunk) * p.chunk_blocks, kb1 = min(p.kblocks, kb0 + p.chunk_blocks);
-        for (int kb = kb0; kb < kb1; ++kb) {
-          if (!kb_needed(kb)) continue;
-          if (!mbar_wait(&empty[stage], phase ^ 1u, cta_err, p.err, 1)) { ok = false; break; }
-          mbar_expect_tx(&full[stage], (uint32_t)(SmemLayout::a_bytes + SmemLayout::b_bytes<BN>()));
-          tma_load_3d(sA + stage * SmemLayout::a_bytes, &tmA, &full[stage], kb * BK, m0, b * p.planes_a + pr.pa);
-          tma_load_3d(sB + stage * SmemLayout::b_bytes<BN>(), &tmB, &full[stage], kb * BK, n0,
-                      b * p.planes_b + pr.pb);
-          ++issued;
-          if (++stage == STAGES) { stage = 0; phase ^= 1u; }
+      for (int kb = 0; kb < p.kblocks && ok; ++kb) {
+        if (!kb_needed(kb)) continue;
+        for (int i = 0; i < p.npairs; ++i) {
+          const TcPair pr = p.pairs[i];
+          if (pr.flags & kPairFirstA) {
+            if (!mbar_wait(&emptyA[sa], pha ^ 1u, cta_err, p.err, 1)) { ok = false; break; }
+            mbar_expect_tx(&fullA[sa], (uint32_t)kTileBytesA);
+            const int pl = MODE == 0 ? pr.pa >> span : pr.pa, k0 = MODE == 0 ? (kb << span) + (pr.pa & span) : kb;
+            tma_load_3d(sA + sa * kTileBytesA, &tmA, &fullA[sa], k0 * BK, m0, b * p.planes_a + pl);
+            ++na;
+            if (++sa == p.slots_a) { sa = 0; pha ^= 1u; }
+          }
+          if (pr.flags & kPairFirstB) {
+            if (!mbar_wait(&emptyB[sb], phb ^ 1u, cta_err, p.err, 1)) { ok = false; break; }
+            mbar_expect_tx(&fullB[sb], (uint32_t)TB);
+            // f32 mode: B's planes from the last to the first
+            const int pl = MODE == 0 ? pr.pb >> span : p.planes_b - 1 - pr.pb;
+            const int k0 = MODE == 0 ? (kb << span) + (pr.pb & span) : kb;
+            tma_load_3d(sB + sb * TB, &tmB, &fullB[sb], k0 * BK, n0, b * p.planes_b + pl);
+            ++nb;
+            if (++sb == p.slots_b) { sb = 0; phb ^= 1u; }
+          }
         }
       }
       if (!ok) {
         // wait (bounded) for the copies still in flight before the CTA exits
-        int st = stage;
-        uint32_t ph = phase;
-        for (int q = 0; q < STAGES && q < issued; ++q) {
-          if (--st < 0) { st = STAGES - 1; ph ^= 1u; }
-          const unsigned long long t0 = now_ns();
-          while (!mbar_try(&full[st], ph) && (long long)(now_ns() - t0) < kWaitNs) {
+        auto settle = [&](uint64_t* full, int slots, int s, uint32_t ph, int issued) {
+          for (int q = 0; q < slots && q < issued; ++q) {
+            if (--s < 0) { s = slots - 1; ph ^= 1u; }
+            const unsigned long long t0 = now_ns();
+            while (!mbar_try(&full[s], ph) && (long long)(now_ns() - t0) < kWaitNs) {
+            }
           }
-        }
+        };
+        settle(fullA, p.slots_a, sa, pha, na);
+        settle(fullB, p.slots_b, sb, phb, nb);
       }
     }
   } else if (warp == MMA_WARP) {
-    if (lane == 0) {
-      int stage = 0;
-      uint32_t phase = 0;
-      bool ok = true;
-      int ls = 0;   // live segments so far (the accumulator ring follows them)
-      for (int si = 0; si < nseg && ok; ++si) {
-        if (!seg_live(si)) continue;
-        const int kb0 = (si % nchunk) * p.chunk_blocks, kb1 = min(p.kblocks, kb0 + p.chunk_blocks);
-        const int buf = ls & 1;
-        {
-          const uint32_t use = (uint32_t)(ls >> 1);
-          if (!mbar_wait(&accempty[buf], (use & 1u) ^ 1u, cta_err, p.err, 2)) { ok = false; break; }
-          tc_fence_after();
-        }
-        ++ls;
+    // the whole warp runs the schedule, so that slots and descriptors stay in
+    // uniform registers; one elected lane issues
+    const bool leader = elect_one();
+    const uint32_t a_lo = (smem_u32(sA) >> 4) | kDescLo, b_lo = (smem_u32(sB) >> 4) | kDescLo;
+    int basea = 0, baseb = 0;           // slots of this K-step's tile 0
+    uint32_t pha = 0, phb = 0;
+    bool ok = true;
+    int buf = 0;                        // accumulator of the current group and its wrap-around parity
+    uint32_t phacc = 1;
+    for (int kb = 0; kb < p.kblocks && ok; ++kb) {
+      if (!kb_needed(kb)) continue;
+      for (int i = 0; i < p.npairs; ++i) {
+        const TcPair pr = p.pairs[i];
+        // tiles enter the rings in the order of their first use, 0, 1, ...
+        int sa = basea + pr.pa, sb = baseb + pr.pb;
+        uint32_t fa = pha, fb = phb;
+        while (sa >= p.slots_a) { sa -= p.slots_a; fa ^= 1u; }
+        while (sb >= p.slots_b) { sb -= p.slots_b; fb ^= 1u; }
+        const bool start = (pr.flags & kPairStart) != 0;
+        if (start) ok = mbar_wait(&accempty[buf], phacc, cta_err, p.err, 2);
+        if (ok && (pr.flags & kPairFirstA)) ok = mbar_wait(&fullA[sa], fa, cta_err, p.err, 3);
+        if (ok && (pr.flags & kPairFirstB)) ok = mbar_wait(&fullB[sb], fb, cta_err, p.err, 3);
+        if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
+        tc_fence_after();
         const uint32_t dt = tmem + (uint32_t)(buf * BN);
-        bool fresh = true;   // the segment's first issued block overwrites the accumulator
-        for (int kb = kb0; kb < kb1; ++kb) {
-          if (!kb_needed(kb)) continue;
-          if (!mbar_wait(&full[stage], phase, cta_err, p.err, 3)) { ok = false; break; }
-          tc_fence_after();
-          const uint64_t ad = sdesc(smem_u32(sA + stage * SmemLayout::a_bytes));
-          const uint64_t bd = sdesc(smem_u32(sB + stage * SmemLayout::b_bytes<BN>()));
+        const uint32_t al = a_lo + sa * (kTileBytesA >> 4), bl = b_lo + sb * (TB >> 4);
+        if (leader) {
 #pragma unroll
-          for (int k = 0; k < BK / 16; ++k) {
-            const bool first = fresh && k == 0;
+          for (int k = 0; k < BK / 16; ++k)
             // +32 bytes of K per instruction: +2 in the descriptor's address field
-            umma(dt, ad + 2 * k, bd + 2 * k, IDESC, first ? 0u : 1u);
-          }
-          umma_commit(&empty[stage]);
-          fresh = false;
-          if (++stage == STAGES) { stage = 0; phase ^= 1u; }
+            umma(dt, sdesc(al + 2 * k), sdesc(bl + 2 * k), IDESC, (start && k == 0) ? 0u : 1u);
+          if (pr.flags & kPairLastA) umma_commit(&emptyA[sa]);
+          if (pr.flags & kPairLastB) umma_commit(&emptyB[sb]);
+          if (pr.flags & kPairEnd) umma_commit(&accfull[buf]);
         }
-        if (ok) umma_commit(&accfull[buf]);
+        __syncwarp();
+        if (pr.flags & kPairEnd) {
+          if (++buf == NACC) { buf = 0; phacc ^= 1u; }
+        }
       }
+      basea += p.planes_a * p.kspan;
+      while (basea >= p.slots_a) { basea -= p.slots_a; pha ^= 1u; }
+      baseb += p.planes_b * p.kspan;
+      while (baseb >= p.slots_b) { baseb -= p.slots_b; phb ^= 1u; }
     }
   } else {
     // ---------------- epilogue warps ----------------
     const int q = warp & 3, h = warp >> 2;
     const int row = m0 + 32 * q + lane;
     const uint32_t lane_addr = tmem + ((uint32_t)(32 * q) << 16);
+    bool ok = true;
+    int g = 0;
     if (MODE == 0) {
-      long long acc[64];
+      long long acc[CW];
 #pragma unroll
-      for (int j = 0; j < 64; ++j) acc[j] = 0;
-      bool ok = true;
-      int ls = 0;
-      for (int si = 0; si < nseg; ++si) {
-        if (!seg_live(si)) continue;
-        const int buf = ls & 1;
-        const uint32_t use = (uint32_t)(ls >> 1);
-        ++ls;
-        ok = __all_sync(0xffffffffu, mbar_wait(&accfull[buf], use & 1u, cta_err, p.err, 4));
-        if (!ok) break;
-        tc_fence_after();
-        const int sh = p.pairs[si / nchunk].shift;
+      for (int j = 0; j < CW; ++j) acc[j] = 0;
+      for (int kb = 0; kb < p.kblocks && ok; ++kb) {
+        if (!kb_needed(kb)) continue;
+        for (int i = 0; i < p.ngroups; ++i, ++g) {
+          const int buf = g % NACC;
+          ok = __all_sync(0xffffffffu, mbar_wait(&accfull[buf], (uint32_t)(g / NACC) & 1u, cta_err, p.err, 4));
+          if (!ok) break;
+          tc_fence_after();
+          const int sh = p.shift[i];
 #pragma unroll
-        for (int part = 0; part < 4; ++part) {
-          uint32_t r[16];
-          tmem_ld16(lane_addr + (uint32_t)(buf * BN + 64 * h + 16 * part), r);
-          tmem_ld_wait();
-          if (part == 3) {
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&accempty[buf]);
-          }
-          if (sh >= 0) {
+          for (int part = 0; part < CW / 16; ++part) {
+            uint32_t r[16];
+            tmem_ld16(lane_addr + (uint32_t)(buf * BN + CW * h + 16 * part), r);
+            tmem_ld_wait();
+            if (part == CW / 16 - 1) {
+              tc_fence_before();
+              __syncwarp();
+              if (lane == 0) mbar_arrive(&accempty[buf]);
+            }
+            if (sh > 30) {
 #pragma unroll
-            for (int j = 0; j < 16; ++j)
-              acc[16 * part + j] += (long long)__float2int_rn(__uint_as_float(r[j])) << sh;
-          } else {
-            // low-order digit groups: rounded to the accumulator's unit (a
-            // plain arithmetic shift would floor, a bias of half a unit per
-            // drain that adds up over long K)
-            const long long half = 1LL << (-sh - 1);
+              for (int j = 0; j < 16; ++j)
+                acc[16 * part + j] += (long long)__float2int_rn(__uint_as_float(r[j])) << sh;
+            } else if (sh >= 0) {
+              // one 32 x 32 + 64-bit multiply-add per sum
+              const int mul = 1 << sh;
 #pragma unroll
-            for (int j = 0; j < 16; ++j)
-              acc[16 * part + j] += ((long long)__float2int_rn(__uint_as_float(r[j])) + half) >> (-sh);
+              for (int j = 0; j < 16; ++j)
+                acc[16 * part + j] += (long long)__float2int_rn(__uint_as_float(r[j])) * mul;
+            } else {
+              // low-order digit groups: rounded to the accumulator's unit (a
+              // plain arithmetic shift would floor, a bias of half a unit per
+              // drain that adds up over long K)
+              const int half = 1 << (-sh - 1);
+#pragma unroll
+              for (int j = 0; j < 16; ++j)
+                acc[16 * part + j] += (__float2int_rn(__uint_as_float(r[j])) + half) >> (-sh);
+            }
           }
         }
       }
       if (ok && row < p.m) {
         const int er = p.ea[(size_t)b * p.m + row] + p.base;
-        const int c0 = (n0 >> 1) + 32 * h;     // first complex column of this warp
+        const int c0 = (n0 >> 1) + CW / 2 * h;     // first complex column of this warp
         double2* out = reinterpret_cast<double2*>(p.c64) + (size_t)b * p.stride_c;
 #pragma unroll
-        for (int j = 0; j < 32; ++j) {
+        for (int j = 0; j < CW / 2; ++j) {
           const int c = c0 + j;
           if (c < p.ncols) {
             const int e = er + p.fb[(size_t)b * p.ncols + c];
@@ -408,42 +434,39 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
         }
       }
     } else {
-      // FP32 mode: every segment (one piece pair over at most 512 of K') is
-      // drained into register accumulators with round-to-nearest adds, so
-      // that long sums of like-signed terms are not left to the tensor
-      // core's accumulator alone
-      float acc[128];
+      // every K-block's sums (384 products) are drained into register
+      // accumulators with round-to-nearest adds, so that long sums of
+      // like-signed terms are not left to the tensor core's accumulator alone
+      float acc[CW];
 #pragma unroll
-      for (int j = 0; j < 128; ++j) acc[j] = 0.f;
-      bool ok = true;
-      int ls = 0;
-      for (int si = 0; si < nseg; ++si) {
-        if (!seg_live(si)) continue;
-        const int buf = ls & 1;
-        const uint32_t use = (uint32_t)(ls >> 1);
-        ++ls;
-        ok = __all_sync(0xffffffffu, mbar_wait(&accfull[buf], use & 1u, cta_err, p.err, 4));
-        if (!ok) break;
-        tc_fence_after();
+      for (int j = 0; j < CW; ++j) acc[j] = 0.f;
+      for (int kb = 0; kb < p.kblocks && ok; ++kb) {
+        if (!kb_needed(kb)) continue;
+        for (int i = 0; i < p.ngroups; ++i, ++g) {
+          const int buf = g % NACC;
+          ok = __all_sync(0xffffffffu, mbar_wait(&accfull[buf], (uint32_t)(g / NACC) & 1u, cta_err, p.err, 4));
+          if (!ok) break;
+          tc_fence_after();
 #pragma unroll
-        for (int part = 0; part < 8; ++part) {
-          uint32_t r[16];
-          tmem_ld16(lane_addr + (uint32_t)(buf * BN + 128 * h + 16 * part), r);
-          tmem_ld_wait();
-          if (part == 7) {
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&accempty[buf]);
+          for (int part = 0; part < CW / 16; ++part) {
+            uint32_t r[16];
+            tmem_ld16(lane_addr + (uint32_t)(buf * BN + CW * h + 16 * part), r);
+            tmem_ld_wait();
+            if (part == CW / 16 - 1) {
+              tc_fence_before();
+              __syncwarp();
+              if (lane == 0) mbar_arrive(&accempty[buf]);
+            }
+#pragma unroll
+            for (int j = 0; j < 16; ++j) acc[16 * part + j] += __uint_as_float(r[j]);
           }
-#pragma unroll
-          for (int j = 0; j < 16; ++j) acc[16 * part + j] += __uint_as_float(r[j]);
         }
       }
       if (ok && row < p.m) {
         float2* out = reinterpret_cast<float2*>(p.c32) + (size_t)b * p.stride_c;
-        const int cbase = (n0 >> 1) + 64 * h;
+        const int cbase = (n0 >> 1) + CW / 2 * h;
 #pragma unroll
-        for (int j = 0; j < 64; ++j) {
+        for (int j = 0; j < CW / 2; ++j) {
           const int c = cbase + j;
           if (c < p.ncols) {
             float2 v = make_float2(p.alpha * acc[2 * j], p.alpha * acc[2 * j + 1]);
@@ -463,7 +486,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
   __syncthreads();
   if (warp == MMA_WARP) {
     tc_fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(tmem_cols<MODE>()));
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols));
   }
 }
 
@@ -516,121 +539,139 @@ __global__ void line_expo_kernel(const T* __restrict__ src, long long sstride, i
   if (lane == 0) expo[gw] = bound_expo(T(0), E);
 }
 
-// Exponents of the rows of a column-major source (thread per row).
+// Exponents of the rows of a column-major source: block of 32 rows, the
+// columns spread over its warps.
 template <class T>
-__global__ void row_expo_kernel(const T* __restrict__ src, long long sstride, int ld, int rows, int cols, int nb,
-                                int* __restrict__ expo) {
-  const size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-  if (t >= (size_t)rows * nb) return;
-  const int b = (int)(t / rows), r = (int)(t % rows);
+__global__ void __launch_bounds__(256) row_expo_kernel(const T* __restrict__ src, long long sstride, int ld, int rows,
+                                                       int cols, int* __restrict__ expo) {
+  __shared__ int part[8][32];
+  const int b = blockIdx.y, r = blockIdx.x * 32 + threadIdx.x;
   const T* s = src + (size_t)b * sstride;
   int E = 0;
-  for (int c = 0; c < cols; ++c) {
-    E = max(E, expo_field(s[2 * ((size_t)c * ld + r)]));
-    E = max(E, expo_field(s[2 * ((size_t)c * ld + r) + 1]));
+  if (r < rows) {
+#pragma unroll 8
+    for (int c = threadIdx.y; c < cols; c += 8) {
+      E = max(E, expo_field(s[2 * ((size_t)c * ld + r)]));
+      E = max(E, expo_field(s[2 * ((size_t)c * ld + r) + 1]));
+    }
   }
-  expo[t] = bound_expo(T(0), E);
+  part[threadIdx.y][threadIdx.x] = E;
+  __syncthreads();
+  if (threadIdx.y == 0 && r < rows) {
+#pragma unroll
+    for (int w = 1; w < 8; ++w) E = max(E, part[w][threadIdx.x]);
+    expo[(size_t)b * rows + r] = bound_expo(T(0), E);
+  }
 }
 
-// Value of plane `pl` of x: digit pl of the fixed-point split (beta bits,
-// W = nplanes * beta) or BF16 piece pl of an FP32 value.
+// x as signed fixed point (W bits of magnitude, truncated) plus the bias that
+// turns its base-256 digits into balanced ones: digit 0 = biased >> 8 (np - 1),
+// in [-256, 256], digit pl = ((biased >> 8 (np - 1 - pl)) & 255) - 128.
 template <class T>
-__device__ __forceinline__ float plane_value(T x, int e, int beta, int W, int pl, bool digits) {
-  if (digits) {
-    const unsigned long long N = fixed_bits(x, e, W);
-    const int d = (int)((N >> (W - beta * (pl + 1))) & ((1ULL << beta) - 1ULL));
-    return x < T(0) ? -(float)d : (float)d;
-  }
-  float r = (float)x;
-  float v = 0.f;
-  for (int i = 0; i <= pl; ++i) {
-    v = __bfloat162float(__float2bfloat16_rn(r));
-    r -= v;
-  }
-  return v;
+__device__ __forceinline__ long long biased_fixed(T x, int e, int nplanes) {
+  const long long m = (long long)fixed_bits(x, e, nplanes * kBeta);
+  long long bias = 0;
+  for (int q = 0; q < nplanes - 1; ++q) bias = (bias << kBeta) + 128;
+  return (x < T(0) ? -m : m) + bias;
 }
+__device__ __forceinline__ float digit_of(long long biased, int nplanes, int pl) {
+  const int sh = kBeta * (nplanes - 1 - pl);
+  return pl == 0 ? (float)(int)(biased >> sh) : (float)((int)((unsigned long long)biased >> sh & 255u) - 128);
+}
+
+// Plane values of one real number, plane after plane: digits, or the BF16
+// pieces of an FP32 value.
+template <class T>
+struct PlaneValue {
+  long long biased;
+  float rest;
+  __device__ __forceinline__ PlaneValue(T x, int e, int nplanes, bool digits)
+      : biased(digits ? biased_fixed(x, e, nplanes) : 0), rest((float)x) {}
+  __device__ __forceinline__ __nv_bfloat16 next(int nplanes, int pl, bool digits) {
+    if (digits) return __float2bfloat16_rn(digit_of(biased, nplanes, pl));
+    const __nv_bfloat16 v = __float2bfloat16_rn(rest);
+    rest -= __bfloat162float(v);
+    return v;
+  }
+};
 
 // Left operand planes: out[b][pl][r][Kp] with columns [0, k) = Re op(A)(r, .),
 // [kp, kp + k) = Im op(A)(r, .), zero elsewhere (Kp = 2 kp).  op(A) = src or
-// src^H; 32 x 32 tiles through shared memory so that reads and writes
-// coalesce in both cases.
+// src^H; tiles of 32 rows by 64 of K through shared memory so that reads and
+// writes (two BF16 a lane) coalesce in both cases.
 template <class T>
 __global__ void __launch_bounds__(256) slice_a_kernel(const T* __restrict__ src, long long sstride, int ld, bool conj,
                                                       int m, int k, int kp, const int* __restrict__ ea,
-                                                      int nplanes, int beta, bool digits,
-                                                      __nv_bfloat16* __restrict__ out) {
-  __shared__ T tre[32][33], tim[32][33];
+                                                      int nplanes, bool digits, __nv_bfloat16* __restrict__ out) {
+  __shared__ T tre[32][65], tim[32][65];
   const int b = blockIdx.z;
-  const int r0 = blockIdx.x * 32, c0 = blockIdx.y * 32;   // rows of op(A), K columns
+  const int r0 = blockIdx.x * 32, c0 = blockIdx.y * 64;   // rows of op(A), K columns
   const int tx = threadIdx.x, ty = threadIdx.y;
   const T* s = src + (size_t)b * sstride;
-  for (int j = ty; j < 32; j += 8) {
-    // tre[r][c] = op(A)(r0 + r, c0 + c)
-    if (!conj) {
+  // tre[r][c] = op(A)(r0 + r, c0 + c)
+  if (!conj) {
+    for (int j = ty; j < 64; j += 8) {
       const int r = r0 + tx, c = c0 + j;
-      T vr = T(0), vi = T(0);
-      if (r < m && c < k) {
-        vr = s[2 * ((size_t)c * ld + r)];
-        vi = s[2 * ((size_t)c * ld + r) + 1];
-      }
-      tre[tx][j] = vr;
-      tim[tx][j] = vi;
-    } else {
-      const int c = c0 + tx, r = r0 + j;
-      T vr = T(0), vi = T(0);
-      if (r < m && c < k) {
-        vr = s[2 * ((size_t)r * ld + c)];
-        vi = -s[2 * ((size_t)r * ld + c) + 1];
-      }
-      tre[j][tx] = vr;
-      tim[j][tx] = vi;
+      const bool in = r < m && c < k;
+      const size_t at = 2 * ((size_t)c * ld + r);
+      tre[tx][j] = in ? s[at] : T(0);
+      tim[tx][j] = in ? s[at + 1] : T(0);
     }
+  } else {
+    for (int j = ty; j < 32; j += 8)
+      for (int x = tx; x < 64; x += 32) {
+        const int r = r0 + j, c = c0 + x;
+        const bool in = r < m && c < k;
+        const size_t at = 2 * ((size_t)r * ld + c);
+        tre[j][x] = in ? s[at] : T(0);
+        tim[j][x] = in ? -s[at + 1] : T(0);
+      }
   }
   __syncthreads();
-  const int W = nplanes * beta;
   const size_t Kp = 2 * (size_t)kp;
   for (int j = ty; j < 32; j += 8) {
-    const int r = r0 + j, c = c0 + tx;
+    const int r = r0 + j, c = c0 + 2 * tx;
     if (r >= m || c >= kp) continue;
-    const T xr = tre[j][tx], xi = tim[j][tx];
     const int e = digits ? ea[(size_t)b * m + r] : 0;
+    PlaneValue<T> x0(tre[j][2 * tx], e, nplanes, digits), x1(tre[j][2 * tx + 1], e, nplanes, digits);
+    PlaneValue<T> y0(tim[j][2 * tx], e, nplanes, digits), y1(tim[j][2 * tx + 1], e, nplanes, digits);
     for (int pl = 0; pl < nplanes; ++pl) {
-      __nv_bfloat16* o = out + (((size_t)b * nplanes + pl) * m + r) * Kp;
-      o[c] = __float2bfloat16_rn(c < k ? plane_value(xr, e, beta, W, pl, digits) : 0.f);
-      o[kp + c] = __float2bfloat16_rn(c < k ? plane_value(xi, e, beta, W, pl, digits) : 0.f);
+      __nv_bfloat16* o = out + (((size_t)b * nplanes + pl) * m + r) * Kp + c;
+      *reinterpret_cast<__nv_bfloat162*>(o) = __nv_bfloat162(x0.next(nplanes, pl, digits), x1.next(nplanes, pl, digits));
+      *reinterpret_cast<__nv_bfloat162*>(o + kp) =
+          __nv_bfloat162(y0.next(nplanes, pl, digits), y1.next(nplanes, pl, digits));
     }
   }
 }
 
 // Right operand planes: out[b][pl][2c + (0|1)][Kp]: row 2c = [Re B(., c) | -Im B(., c)],
-// row 2c+1 = [Im B(., c) | Re B(., c)]; thread per (column, K index).
+// row 2c+1 = [Im B(., c) | Re B(., c)]; thread per column and two K indices.
 template <class T>
 __global__ void slice_b_kernel(const T* __restrict__ src, long long sstride, int ld, int k, int n, int kp,
-                               const int* __restrict__ fb, int nplanes, int beta, bool digits, int nb,
+                               const int* __restrict__ fb, int nplanes, bool digits, int nb,
                                __nv_bfloat16* __restrict__ out) {
-  const size_t per = (size_t)kp * n, total = per * nb;
-  const int W = nplanes * beta;
+  const int half = kp >> 1;
+  const size_t per = (size_t)half * n, total = per * nb;
   const size_t Kp = 2 * (size_t)kp;
   for (size_t idx = blockIdx.x * (size_t)blockDim.x + threadIdx.x; idx < total;
        idx += (size_t)gridDim.x * blockDim.x) {
     const int b = (int)(idx / per);
-    const size_t q = idx % per;
-    const int r = (int)(q % kp), c = (int)(q / kp);
-    const T* s = src + (size_t)b * sstride;
-    T xr = T(0), xi = T(0);
-    if (r < k) {
-      xr = s[2 * ((size_t)c * ld + r)];
-      xi = s[2 * ((size_t)c * ld + r) + 1];
-    }
+    const size_t q = idx - (size_t)b * per;
+    const int c = (int)(q / half), r = 2 * (int)(q - (size_t)c * half);
+    const T* s = src + (size_t)b * sstride + 2 * ((size_t)c * ld + r);
+    const T v[4] = {r < k ? s[0] : T(0), r < k ? s[1] : T(0), r + 1 < k ? s[2] : T(0), r + 1 < k ? s[3] : T(0)};
     const int e = digits ? fb[(size_t)b * n + c] : 0;
+    PlaneValue<T> x0(v[0], e, nplanes, digits), y0(v[1], e, nplanes, digits);
+    PlaneValue<T> x1(v[2], e, nplanes, digits), y1(v[3], e, nplanes, digits);
     for (int pl = 0; pl < nplanes; ++pl) {
-      const float vr = r < k ? plane_value(xr, e, beta, W, pl, digits) : 0.f;
-      const float vi = r < k ? plane_value(xi, e, beta, W, pl, digits) : 0.f;
-      __nv_bfloat16* o = out + (((size_t)b * nplanes + pl) * 2 * n + 2 * (size_t)c) * Kp;
-      o[r] = __float2bfloat16_rn(vr);
-      o[kp + r] = __float2bfloat16_rn(-vi);
-      o[Kp + r] = __float2bfloat16_rn(vi);
-      o[Kp + kp + r] = __float2bfloat16_rn(vr);
+      const __nv_bfloat162 re(x0.next(nplanes, pl, digits), x1.next(nplanes, pl, digits));
+      const __nv_bfloat162 im(y0.next(nplanes, pl, digits), y1.next(nplanes, pl, digits));
+      __nv_bfloat162* o =
+          reinterpret_cast<__nv_bfloat162*>(out + (((size_t)b * nplanes + pl) * 2 * n + 2 * (size_t)c) * Kp + r);
+      o[0] = re;
+      o[half] = __hneg2(im);
+      o[kp] = im;
+      o[kp + half] = re;
     }
   }
 }
@@ -733,6 +774,37 @@ int make_map(CUtensorMap* map, const void* base, size_t Kp, size_t rows, size_t 
 int* g_err = nullptr;   // device error word shared by the launches of this process
 std::mutex g_err_mu;
 
+// First / last uses of the tiles, and the tile slots.  The slots cover what a
+// K-step keeps live plus what is staged ahead, 224 KB in all: fixed mode 14 of
+// 16 KB (7 + 7 digits in one K-block: all live at once; 3 + 6 digits in two
+// K-blocks: the three-digit operand's six tiles live throughout, a window of
+// six of the other's); f32 mode 6 of 16 KB and 4 of 32 KB.
+void plan_pairs(TcParams& p, int mode) {
+  for (int i = 0; i < p.npairs; ++i) {
+    TcPair& pr = p.pairs[i];
+    bool firstA = true, firstB = true, lastA = true, lastB = true;
+    for (int j = 0; j < p.npairs; ++j) {
+      if (j < i) {
+        firstA &= p.pairs[j].pa != pr.pa;
+        firstB &= p.pairs[j].pb != pr.pb;
+      } else if (j > i) {
+        lastA &= p.pairs[j].pa != pr.pa;
+        lastB &= p.pairs[j].pb != pr.pb;
+      }
+    }
+    pr.flags = (int16_t)((pr.flags & (kPairStart | kPairEnd)) | (firstA ? kPairFirstA : 0) | (firstB ? kPairFirstB : 0) |
+                         (lastA ? kPairLastA : 0) | (lastB ? kPairLastB : 0));
+  }
+  if (p.kspan == 2) p.kblocks = (p.kblocks + 1) / 2;     // a step past K' reads zeros
+  if (mode == 0) {
+    p.slots_a = p.planes_a < p.planes_b ? 6 : p.planes_a > p.planes_b ? 8 : 7;
+    p.slots_b = 14 - p.slots_a;
+  } else {
+    p.slots_a = 6;
+    p.slots_b = 4;
+  }
+}
+
 int launch(olc_context* ctx, int mode, const void* dA, const void* dB, int planes_a, int planes_b, size_t Kp,
            int m, int nreal, int nb, TcParams p, int stage) {
   cudaStream_t st = ctx->stream;
@@ -755,19 +827,19 @@ int launch(olc_context* ctx, int mode, const void* dA, const void* dB, int plane
   p.kblocks = (int)(Kp / BK);
   p.kp = (int)(Kp / 2);
   p.err = g_err;
+  plan_pairs(p, mode);
   const dim3 grid((unsigned)(p.nmt * p.nnt), (unsigned)nb);
+  const int smem = smem_total(mode, p.slots_a, p.slots_b);
   if (mode == 0) {
-    const int smem = SmemLayout::total<128>();
     if ((s = cuda_check(cudaFuncSetAttribute(tc_gemm_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem),
                         "tc smem")))
       return s;
-    tc_gemm_kernel<0><<<grid, NUM_THREADS, smem, st>>>(ta, tb, p);
+    tc_gemm_kernel<0><<<grid, num_threads<0>(), smem, st>>>(ta, tb, p);
   } else {
-    const int smem = SmemLayout::total<256>();
     if ((s = cuda_check(cudaFuncSetAttribute(tc_gemm_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem),
                         "tc smem")))
       return s;
-    tc_gemm_kernel<1><<<grid, NUM_THREADS, smem, st>>>(ta, tb, p);
+    tc_gemm_kernel<1><<<grid, num_threads<1>(), smem, st>>>(ta, tb, p);
   }
   count_launch();
   double frac = 1.0;
@@ -778,13 +850,13 @@ int launch(olc_context* ctx, int mode, const void* dA, const void* dB, int plane
         done += p.herm_upper ? ((nt * BN) / 2 + BN / 2 - 1 >= mt * BM) : ((nt * BN) / 2 <= mt * BM + BM - 1);
     frac = (double)done / ((double)p.nmt * p.nnt);
   }
-  add_work(ctx, stage, 2.0 * m * (double)nreal * (double)Kp * p.npairs * nb * frac, 0.0);
+  add_work(ctx, stage, 2.0 * m * (double)nreal * (double)Kp * (p.npairs / p.kspan) * nb * frac, 0.0);
   return cuda_check(cudaGetLastError(), "tc_gemm launch");
 }
 
 }  // namespace
 
-// Kept-digit plan of a fixed-point product: beta = 7, na / nb digits of A / B,
+// Kept-digit plan of a fixed-point product: na / nb digits of A / B,
 // pairs (s, t) with s + t <= T kept, T the smallest with the dropped part
 // below 2^-(prec + 2) of the scale product.
 void fixed_plan(int bits_a, int bits_b, int prec, int* na, int* nbd, int* T) {
@@ -815,18 +887,30 @@ int zgemm_fixed(olc_context* ctx, int m, int n, int k, const TA* A, long long sA
   fixed_plan(bits_a, bits_b, std::max(bits_a, bits_b), &na, &nbd, &T);
   const int kp = (k + 31) & ~31;
   const size_t Kp = 2 * (size_t)kp;
-  // FP32-exact segments: at most kChunkK of K' per drain
-  std::vector<TcPair> pairs;
-  for (int d = 0; d <= T; ++d)
-    for (int s = 0; s < na; ++s) {
-      const int t = d - s;
-      if (t >= 0 && t < nbd) pairs.push_back(TcPair{(int8_t)s, (int8_t)t, 0});
-    }
-  if ((int)pairs.size() > kMaxPairs) return fail(OLC_ERR_UNSUPPORTED, "fixed-point product: too many digit pairs");
+  // one group per weight s + t = d <= T, its pairs with A's new plane first and
+  // B's last (planes enter in the order 0, 1, ..)
+  TcParams plan{};
   // 64-bit fixed point: unit 2^(L - beta (T + 2)) of the scale product
   const double mag = kBeta * T + 2 * kBeta + std::log2(1.03 * (double)Kp);
   const int L = std::max(0, (int)std::ceil(mag - 62.0));
-  for (auto& pr : pairs) pr.shift = (int16_t)(kBeta * (T - pr.pa - pr.pb) - L);
+  // Up to three pairs a weight, the group's sum stays an exact integer over two
+  // K-blocks (128 (2 2^15 + 2^14) < 2^24): half the drains, which bound this mode
+  // (a drain of the 128 x 128 tile takes the epilogue 1600 clocks, three pairs of
+  // one K-block the tensor cores 950).
+  plan.kspan = std::min(na, nbd) <= 3 ? 2 : 1;
+  for (int d = 0; d <= T; ++d) {
+    const int first = plan.npairs;
+    for (int s = std::min(d, na - 1); s >= 0 && d - s < nbd; --s)
+      for (int q = 0; q < plan.kspan; ++q) {
+        if (plan.npairs == kMaxPairs || plan.ngroups == kMaxGroups)
+          return fail(OLC_ERR_UNSUPPORTED, "fixed-point product: too many digit pairs");
+        plan.pairs[plan.npairs++] = TcPair{(int8_t)(plan.kspan * s + q), (int8_t)(plan.kspan * (d - s) + q), 0};
+      }
+    if (plan.npairs == first) continue;
+    plan.pairs[first].flags |= kPairStart;
+    plan.pairs[plan.npairs - 1].flags |= kPairEnd;
+    plan.shift[plan.ngroups++] = (int16_t)(kBeta * (T - d) - L);
+  }
   // batch chunk: digit planes below ~8 GB
   const size_t per_b = 2 * Kp * ((size_t)na * m + (size_t)nbd * 2 * n);
   const int chunk = (int)std::max<size_t>(1, std::min<size_t>(nb, (8ULL << 30) / std::max<size_t>(per_b, 1)));
@@ -847,14 +931,13 @@ int zgemm_fixed(olc_context* ctx, int m, int n, int k, const TA* A, long long sA
     if (conjA)
       line_expo_kernel<TA><<<(int)(((size_t)m * cb * 32 + 255) / 256), 256, 0, st>>>(Ab, sA, lda, k, m, cb, ea);
     else
-      row_expo_kernel<TA><<<(int)(((size_t)m * cb + 255) / 256), 256, 0, st>>>(Ab, sA, lda, m, k, cb, ea);
+      row_expo_kernel<TA><<<dim3((m + 31) / 32, cb), dim3(32, 8), 0, st>>>(Ab, sA, lda, m, k, ea);
     line_expo_kernel<TB><<<(int)(((size_t)n * cb * 32 + 255) / 256), 256, 0, st>>>(Bb, sB, ldb, k, n, cb, fb);
-    slice_a_kernel<TA><<<dim3((m + 31) / 32, (kp + 31) / 32, cb), dim3(32, 8), 0, st>>>(
-        Ab, sA, lda, conjA, m, k, kp, ea, na, kBeta, true, wa);
-    slice_b_kernel<TB><<<grid_of((size_t)kp * n * cb), 256, 0, st>>>(Bb, sB, ldb, k, n, kp, fb, nbd, kBeta, true,
-                                                                     cb, wb);
+    slice_a_kernel<TA><<<dim3((m + 31) / 32, (kp + 63) / 64, cb), dim3(32, 8), 0, st>>>(
+        Ab, sA, lda, conjA, m, k, kp, ea, na, true, wa);
+    slice_b_kernel<TB><<<grid_of((size_t)kp / 2 * n * cb), 256, 0, st>>>(Bb, sB, ldb, k, n, kp, fb, nbd, true, cb, wb);
     scope.add_launches(5);
-    TcParams p{};
+    TcParams p = plan;
     p.m = m;
     p.ncols = n;
     p.ldc = m;
@@ -863,9 +946,6 @@ int zgemm_fixed(olc_context* ctx, int m, int n, int k, const TA* A, long long sA
     p.ea = ea;
     p.fb = fb;
     p.base = L - kBeta * (T + 2);
-    p.npairs = (int)pairs.size();
-    for (size_t i = 0; i < pairs.size(); ++i) p.pairs[i] = pairs[i];
-    p.chunk_blocks = kChunkK / BK;
     p.herm_upper = hermitian ? 1 : 0;
     if ((s = launch(ctx, 0, wa, wb, na, nbd, Kp, m, 2 * n, cb, p, stage))) return s;
     if (hermitian) {
@@ -887,11 +967,23 @@ int cgemm_f32(olc_context* ctx, int m, int n, int k, const float* A, long long s
   cudaStream_t st = ctx->stream;
   const int kp = (k + 31) & ~31;
   const size_t Kp = 2 * (size_t)kp;
-  // piece pairs by weight: the six down to 2^-16, and with OLC_F32_PAIRS=9 the
-  // three of weight 2^-24 and below as well
-  static const int8_t pairs[9][2] = {{0, 0}, {0, 1}, {1, 0}, {1, 1}, {0, 2}, {2, 0}, {1, 2}, {2, 1}, {2, 2}};
-  int npairs = 6;
-  if (const char* v = std::getenv("OLC_F32_PAIRS")) npairs = std::atoi(v) == 9 ? 9 : 6;
+  // the six piece pairs of weight 2^-16 and above, and with OLC_F32_PAIRS=9 the
+  // three below as well: one plane of B (the wide tile) after the other, the
+  // low-order one first, so that a slot of B is free again after its own pairs
+  // (the second index counts B's planes from the last: pairs (a, 2 - b))
+  static const int8_t six[6][2] = {{0, 0}, {0, 1}, {1, 1}, {0, 2}, {1, 2}, {2, 2}};
+  static const int8_t nine[9][2] = {{0, 0}, {1, 0}, {2, 0}, {0, 1}, {1, 1}, {2, 1}, {0, 2}, {1, 2}, {2, 2}};
+  TcParams plan{};
+  const char* pv = std::getenv("OLC_F32_PAIRS");
+  plan.npairs = pv && std::atoi(pv) == 9 ? 9 : 6;
+  for (int i = 0; i < plan.npairs; ++i) {
+    const int8_t* q = plan.npairs == 9 ? nine[i] : six[i];
+    plan.pairs[i] = TcPair{q[0], q[1], 0};
+  }
+  plan.pairs[0].flags |= kPairStart;
+  plan.pairs[plan.npairs - 1].flags |= kPairEnd;
+  plan.ngroups = 1;
+  plan.kspan = 1;
   const size_t per_b = 2 * Kp * 3 * ((size_t)m + 2 * (size_t)n);
   const int chunk = (int)std::max<size_t>(1, std::min<size_t>(nb, (8ULL << 30) / std::max<size_t>(per_b, 1)));
   __nv_bfloat16 *wa = nullptr, *wb = nullptr;
@@ -905,15 +997,15 @@ int cgemm_f32(olc_context* ctx, int m, int n, int k, const float* A, long long s
     const int cb = std::min(chunk, nb - b0);
     const float* Ab = A + (size_t)b0 * sA;
     const float* Bb = B + (size_t)b0 * sB;
-    slice_a_kernel<float><<<dim3((m + 31) / 32, (kp + 31) / 32, cb), dim3(32, 8), 0, st>>>(
-        Ab, sA, lda, conjA, m, k, kp, nullptr, 3, 0, false, wa);
+    slice_a_kernel<float><<<dim3((m + 31) / 32, (kp + 63) / 64, cb), dim3(32, 8), 0, st>>>(
+        Ab, sA, lda, conjA, m, k, kp, nullptr, 3, false, wa);
     if (conjB)
       slice_bh_kernel<<<dim3((n + 31) / 32, (kp + 31) / 32, cb), dim3(32, 8), 0, st>>>(Bb, sB, ldb, k, n, kp, wb);
     else
-      slice_b_kernel<float><<<grid_of((size_t)kp * n * cb), 256, 0, st>>>(Bb, sB, ldb, k, n, kp, nullptr, 3, 0, false,
-                                                                          cb, wb);
+      slice_b_kernel<float><<<grid_of((size_t)kp / 2 * n * cb), 256, 0, st>>>(Bb, sB, ldb, k, n, kp, nullptr, 3, false,
+                                                                              cb, wb);
     scope.add_launches(2);
-    TcParams p{};
+    TcParams p = plan;
     p.m = m;
     p.ncols = n;
     p.ldc = ldc;
@@ -921,9 +1013,6 @@ int cgemm_f32(olc_context* ctx, int m, int n, int k, const float* A, long long s
     p.c32 = C + (size_t)b0 * sC;
     p.alpha = alpha;
     p.beta = beta;
-    p.npairs = npairs;
-    for (int i = 0; i < npairs; ++i) p.pairs[i] = TcPair{pairs[i][0], pairs[i][1], 0};
-    p.chunk_blocks = 512 / BK;
     p.lower_only = lower ? 1 : 0;
     p.tri_a_upper = (tri & kTriAUpper) != 0;
     p.tri_a_lower = (tri & kTriALower) != 0;

@@ -8,15 +8,20 @@
 namespace olc {
 namespace tc {
 
-constexpr int kBeta = 8;         // bits per digit of the fixed-point split (|d| <= 255, exact in BF16)
+constexpr int kBeta = 8;         // bits per digit of the fixed-point split (exact in BF16)
 constexpr int kMaxPairs = 96;    // digit pairs (or BF16-piece pairs) per launch
+constexpr int kMaxGroups = 24;   // groups of pairs that share an accumulator
 
-// One operand-plane pair of a launch; shift: int64 shift of its drained sums
-// (fixed mode, negative = right shift).
+// One pair of operand tiles of a launch, in the order the pairs run within a
+// K-step of kspan K-blocks; pa, pb: tiles in the order of their first use in the
+// step (tile j = plane j / kspan of K-block j % kspan of the step).  flags: kPair*.
 struct TcPair {
   int8_t pa, pb;
-  int16_t shift;
+  int16_t flags;
 };
+constexpr int kPairFirstA = 1, kPairFirstB = 2;   // first use of the tile in the K-step
+constexpr int kPairLastA = 4, kPairLastB = 8;     // last use
+constexpr int kPairStart = 16, kPairEnd = 32;     // first / last pair of its group
 
 // Launch parameters (passed by value: no host memory is read at run time,
 // so launches can be captured into a CUDA graph).
@@ -31,13 +36,16 @@ struct TcParams {
   int base;                     // fixed mode: output scale 2^(ea + fb + base)
   int planes_a, planes_b;       // planes per batch entry
   int nmt, nnt;                 // tiles
-  int npairs, kblocks, chunk_blocks;   // segments: pairs x ceil(kblocks / chunk_blocks) K chunks
+  int npairs, ngroups, kblocks;
+  int kspan;                    // K-blocks per step: 1, or 2 (kblocks counts steps)
+  int slots_a, slots_b;         // shared-memory tile slots
   int herm_upper;               // Hermitian result: tiles wholly below the diagonal are skipped
   int lower_only;               // f32 mode: tiles wholly above the diagonal are skipped
   int kp;                       // complex K per half of K' (K' = 2 kp)
   int tri_a_upper, tri_a_lower, tri_b_upper;   // triangular operands: zero K blocks skipped
   int* err;                     // device error word (expired waits)
   TcPair pairs[kMaxPairs];
+  int16_t shift[kMaxGroups];    // fixed mode: int64 shift of a group's drained sums (negative: right)
 };
 
 // FP64-accurate complex product C[b] = op(A[b]) B[b] (m x n, column-major,
