@@ -31,61 +31,80 @@ namespace {
 // combine, flush and pack; optionally also emit the full upper matrix (+ add)
 struct PackArgs {
   const double* vv;      // [nk][nv][nv]
-  const double* X;       // S_cv^H O_cv          (nullptr when nc == 0)
-  const double* Y;       // S_cv^H O_cc S_cv
+  const double* X;       // S_cv^H (O_cv - O_cc S_cv / 2)   (unused when nc == 0)
   const double* add;     // optional full upper matrix added after the flush
   double* packed;        // [nk][plen][2] or nullptr
   double* full;          // [nk][nv][nv] upper, or nullptr
   int nv;
   int nk;
   int nc;
-  int is_overlap;
 };
 
-__global__ void ortho_pack_kernel(PackArgs a) {
-  const size_t plen = (size_t)a.nv * (a.nv + 1) / 2;
-  const size_t total = plen * a.nk;
-  for (size_t idx = blockIdx.x * (size_t)blockDim.x + threadIdx.x; idx < total;
-       idx += (size_t)gridDim.x * blockDim.x) {
-    const int k = (int)(idx / plen);
-    const size_t r = idx % plen;
-    // column i, row j <= i with r = i(i+1)/2 + j
-    int i = (int)((sqrt(8.0 * (double)r + 1.0) - 1.0) * 0.5);
-    while ((size_t)i * (i + 1) / 2 > r) --i;
-    while ((size_t)(i + 1) * (i + 2) / 2 <= r) ++i;
-    const int j = (int)(r - (size_t)i * (i + 1) / 2);
-    const size_t nn = (size_t)a.nv * a.nv;
-    const size_t off = (size_t)k * nn + (size_t)i * a.nv + j;   // (row j, col i)
-    double re = a.vv[2 * off], im = a.vv[2 * off + 1];
+constexpr int kPackTile = 32;
+
+// Bound by memory: vv and X read once, the packed operator written once.  A
+// block takes tiles of 32 columns x 32 rows of the upper triangle and turns
+// X's mirror tile in shared memory, so every access runs along columns.  The
+// block finds its tile once in FP32; an FP64 square root per element (1/64 of
+// the FP32 rate) and the strided mirror reads took 2.1 ms for 19 operators of
+// order 832 at 8 k-points, this form 0.78 ms.
+__global__ void __launch_bounds__(256) ortho_pack_kernel(PackArgs a) {
+  __shared__ double2 mirror[kPackTile][kPackTile + 1];
+  const int nt = (a.nv + kPackTile - 1) / kPackTile;
+  const long long ntri = (long long)nt * (nt + 1) / 2, total = ntri * a.nk;
+  const size_t plen = (size_t)a.nv * (a.nv + 1) / 2, nn = (size_t)a.nv * a.nv;
+  const int lane = threadIdx.x & 31, row0 = threadIdx.x >> 5;
+  const double2* X = reinterpret_cast<const double2*>(a.X);
+  const double2* add = reinterpret_cast<const double2*>(a.add);
+  double2* full = reinterpret_cast<double2*>(a.full);
+  for (long long b = blockIdx.x; b < total; b += gridDim.x) {
+    const size_t k = (size_t)(b / ntri);
+    const int r = (int)(b % ntri);
+    int ti = (int)((sqrtf(8.f * (float)r + 1.f) - 1.f) * 0.5f);
+    while (ti * (ti + 1) / 2 > r) --ti;
+    while ((ti + 1) * (ti + 2) / 2 <= r) ++ti;
+    const int i0 = ti * kPackTile, j0 = (r - ti * (ti + 1) / 2) * kPackTile;
     if (a.nc) {
-      const double xr = a.X[2 * off], xi = a.X[2 * off + 1];
-      if (a.is_overlap) {   // zherk('U','C',-2)
-        re -= 2.0 * xr;
-        im -= 2.0 * xi;
-      } else {              // zher2k('U','C',-1): X + X^H
-        const size_t offT = (size_t)k * nn + (size_t)j * a.nv + i;
-        re -= xr + a.X[2 * offT];
-        im -= xi - a.X[2 * offT + 1];
-      }
-      if (i == j) im = 0.0;
-      re += a.Y[2 * off];
-      im += a.Y[2 * off + 1];
-      if (fabs(re) < 1.0e-10) re = 0.0;
-      if (fabs(im) < 1.0e-10) im = 0.0;
+      __syncthreads();                       // the last tile's mirror is read
+      for (int q = row0; q < kPackTile; q += 8)
+        if (j0 + q < a.nv && i0 + lane < a.nv)
+          mirror[q][lane] = X[k * nn + (size_t)(j0 + q) * a.nv + i0 + lane];   // (row i, col j)
+      __syncthreads();
     }
-    if (a.packed) {
-      a.packed[2 * idx] = re;
-      a.packed[2 * idx + 1] = im;
-    }
-    if (a.full) {
-      if (a.add) {
-        re += a.add[2 * off];
-        im += a.add[2 * off + 1];
+    for (int q = row0; q < kPackTile; q += 8) {
+      const int i = i0 + q, j = j0 + lane;   // column i, row j <= i
+      if (i >= a.nv || j > i) continue;
+      const size_t off = k * nn + (size_t)i * a.nv + j;
+      double2 v = make_double2(a.vv[2 * off], a.vv[2 * off + 1]);   // the caller's: any 8-byte address
+      if (a.nc) {   // - (X + X^H)
+        const double2 x = X[off], m = mirror[lane][q];
+        v.x -= x.x + m.x;
+        v.y -= x.y - m.y;
+        if (i == j) v.y = 0.0;
+        if (fabs(v.x) < 1.0e-10) v.x = 0.0;
+        if (fabs(v.y) < 1.0e-10) v.y = 0.0;
       }
-      a.full[2 * off] = re;
-      a.full[2 * off + 1] = im;
+      if (a.packed) {
+        double* p = a.packed + 2 * (k * plen + (size_t)i * (i + 1) / 2 + j);
+        p[0] = v.x;
+        p[1] = v.y;
+      }
+      if (full) {
+        if (add) {
+          const double2 w = add[off];
+          v.x += w.x;
+          v.y += w.y;
+        }
+        full[off] = v;
+      }
     }
   }
+}
+
+// W = O_cv - W / 2 with W = O_cc S_cv on entry
+__global__ void core_fold_kernel(const double* __restrict__ cv, double* __restrict__ w, size_t len) {
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < len; i += (size_t)gridDim.x * blockDim.x)
+    w[i] = cv[i] - 0.5 * w[i];
 }
 
 // packed [nk][plen][2] -> full Hermitian [nk][n][n] (both triangles)
@@ -161,49 +180,51 @@ int grid_for(size_t n) {
 
 }  // namespace
 
-// Orthogonalise one operator for all k.  vv/cv/cc are the operator's blocks,
-// scv is S_cv.  Writes packed and/or full (upper, with `add` added).
+// Orthogonalise one operator for all k.  vv/cv/cc are the operator's blocks
+// (cc Hermitian, as an operator's core block is), scv is S_cv.  Writes packed
+// and/or full (upper, with `add` added).
+//   S_cv^H O_cv + O_cv^H S_cv - S_cv^H O_cc S_cv = X + X^H,
+//   X = S_cv^H (O_cv - O_cc S_cv / 2),
+// and for the overlap, O_cv = S_cv, the same: one product of order nv besides
+// O_cc S_cv where the separate terms take two (with the pack kernel below,
+// 19 operators of order 832 at 8 k-points: set-up 104 -> 90 ms).
 int ortho_pack_ex(olc_context* ctx, bool is_overlap, const double* vv, const double* cv,
                   const double* cc, const double* scv, double* packed, double* full,
                   const double* add) {
   const int nv = ctx->dims.vale_dim, nc = ctx->dims.core_dim, nk = ctx->dims.num_kpoints;
   int st;
   if (nc) {
-    const size_t nn = (size_t)nv * nv;
+    const size_t nn = (size_t)nv * nv, ncv = 2 * (size_t)nv * nc * nk;
     if (!ctx->d_work_x) {
       if ((st = dalloc(ctx, &ctx->d_work_x, 2 * nn * nk))) return st;
-      if ((st = dalloc(ctx, &ctx->d_work_y, 2 * nn * nk))) return st;
-      if ((st = dalloc(ctx, &ctx->d_work_w, 2 * (size_t)nv * nc * nk))) return st;
+      if ((st = dalloc(ctx, &ctx->d_work_w, ncv))) return st;
     }
-    // the three products on the tensor cores, FP64-accurate (split digits,
+    // both products on the tensor cores, FP64-accurate (split digits,
     // olc_ozaki.cu); OLC_ORTHO_BITS lowers the bits kept per operand
     int bits = 53;
     if (const char* v = std::getenv("OLC_ORTHO_BITS")) bits = std::max(24, std::min(53, std::atoi(v)));
-    const long long sCV = 2LL * nc * nv, sCC = 2LL * nc * nc, sW = 2LL * nv * nc;
-    // X = S_cv^H O_cv
-    if ((st = ozaki_zgemm<double, double>(ctx, nv, nv, nc, scv, sCV, nc, true, bits, is_overlap ? scv : cv,
-                                          sCV, nc, bits, ctx->d_work_x, nk, OLC_STAGE_ORTHO))) return st;
-    // W = S_cv^H O_cc
-    if ((st = ozaki_zgemm<double, double>(ctx, nv, nc, nc, scv, sCV, nc, true, bits, cc, sCC, nc, bits,
+    const long long sCV = 2LL * nc * nv, sCC = 2LL * nc * nc;
+    if ((st = ozaki_zgemm<double, double>(ctx, nc, nv, nc, cc, sCC, nc, false, bits, scv, sCV, nc, bits,
                                           ctx->d_work_w, nk, OLC_STAGE_ORTHO))) return st;
-    // Y = W S_cv
-    if ((st = ozaki_zgemm<double, double>(ctx, nv, nv, nc, ctx->d_work_w, sW, nv, false, bits, scv, sCV, nc,
-                                          bits, ctx->d_work_y, nk, OLC_STAGE_ORTHO))) return st;
+    {
+      StageScope scope(ctx, OLC_STAGE_ORTHO);
+      core_fold_kernel<<<grid_for(ncv), 256, 0, ctx->stream>>>(is_overlap ? scv : cv, ctx->d_work_w, ncv);
+    }
+    if ((st = ozaki_zgemm<double, double>(ctx, nv, nv, nc, scv, sCV, nc, true, bits, ctx->d_work_w, sCV, nc,
+                                          bits, ctx->d_work_x, nk, OLC_STAGE_ORTHO))) return st;
   }
   PackArgs a;
   a.vv = vv;
   a.X = ctx->d_work_x;
-  a.Y = ctx->d_work_y;
   a.add = add;
   a.packed = packed;
   a.full = full;
   a.nv = nv;
   a.nk = nk;
   a.nc = nc;
-  a.is_overlap = is_overlap ? 1 : 0;
-  const size_t total = (size_t)nv * (nv + 1) / 2 * nk;
+  const size_t nt = (nv + kPackTile - 1) / kPackTile;
   StageScope scope(ctx, OLC_STAGE_ORTHO);
-  ortho_pack_kernel<<<grid_for(total), 256, 0, ctx->stream>>>(a);
+  ortho_pack_kernel<<<(int)std::min<size_t>(nt * (nt + 1) / 2 * nk, 152 * 32), 256, 0, ctx->stream>>>(a);
   return cuda_check(cudaGetLastError(), "ortho_pack_kernel");
 }
 
