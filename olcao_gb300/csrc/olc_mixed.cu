@@ -614,43 +614,105 @@ __global__ void loewdin_prep_kernel(const double* __restrict__ Hh, const double*
   }
 }
 
-// F = -E/2 + (3/8) E2   (in place in E2)
-__global__ void loewdin_f_kernel(const float* __restrict__ E, float* __restrict__ E2, size_t n2) {
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n2;
-       i += (size_t)gridDim.x * blockDim.x)
-    E2[i] = -0.5f * E[i] + 0.375f * E2[i];
+// Tile b of a batch's lower triangles: 32 rows i0.. by 32 columns j0.. <= i0
+// of matrix k, nt tiles a side (the tile's index within the triangle is below
+// 2^24: exact in FP32 up to the correction).
+struct LowerTile {
+  size_t k;
+  int i0, j0;
+};
+__device__ __forceinline__ LowerTile lower_tile(long long b, int nt) {
+  const long long ntri = (long long)nt * (nt + 1) / 2;
+  const int r = (int)(b % ntri);
+  int ti = (int)((sqrtf(8.f * (float)r + 1.f) - 1.f) * 0.5f);
+  while (ti * (ti + 1) / 2 > r) --ti;
+  while ((ti + 1) * (ti + 2) / 2 <= r) ++ti;
+  return LowerTile{(size_t)(b / ntri), ti * 32, (r - ti * (ti + 1) / 2) * 32};
 }
 
-// out (FP64) = base (FP64) + add (FP32); optional FP32 copy of the sum
-__global__ void add_f32_kernel(double* __restrict__ out, const double* __restrict__ base,
-                               const float* __restrict__ add, float* __restrict__ copy32,
+// F = -E/2 + (3/8) E2 in place in E2, whose lower tiles alone are given (the
+// square of a Hermitian matrix); F's upper triangle is the mirror of its
+// lower one.
+__global__ void __launch_bounds__(256) loewdin_f_kernel(const float2* __restrict__ E, float2* __restrict__ E2, int n,
+                                                        int nk) {
+  __shared__ float2 tile[32][33];
+  const int nt = (n + 31) / 32, lane = threadIdx.x & 31, row0 = threadIdx.x >> 5;
+  const long long total = (long long)nt * (nt + 1) / 2 * nk;
+  for (long long b = blockIdx.x; b < total; b += gridDim.x) {
+    const LowerTile t = lower_tile(b, nt);
+    const float2* Ek = E + t.k * n * n;
+    float2* Fk = E2 + t.k * n * n;
+    __syncthreads();                          // the last tile's mirror is written
+    for (int q = row0; q < 32; q += 8) {
+      const int i = t.i0 + lane, j = t.j0 + q;
+      if (i < n && j <= i) {
+        const size_t off = (size_t)j * n + i;
+        const float2 e = Ek[off], e2 = Fk[off];
+        const float2 f = make_float2(-0.5f * e.x + 0.375f * e2.x, i == j ? 0.f : -0.5f * e.y + 0.375f * e2.y);
+        Fk[off] = f;
+        tile[q][lane] = f;
+      }
+    }
+    __syncthreads();
+    for (int q = row0; q < 32; q += 8) {
+      const int i = t.i0 + q, j = t.j0 + lane;
+      if (i < n && j < i) Fk[(size_t)i * n + j] = make_float2(tile[lane][q].x, -tile[lane][q].y);
+    }
+  }
+}
+
+// H (FP64) := H + T (FP32) for a Hermitian sum: lower tiles read, both
+// triangles written.
+__global__ void __launch_bounds__(256) add_hermitian_kernel(double2* __restrict__ H, const float2* __restrict__ T,
+                                                            int n, int nk) {
+  __shared__ double2 tile[32][33];
+  const int nt = (n + 31) / 32, lane = threadIdx.x & 31, row0 = threadIdx.x >> 5;
+  const long long total = (long long)nt * (nt + 1) / 2 * nk;
+  for (long long b = blockIdx.x; b < total; b += gridDim.x) {
+    const LowerTile t = lower_tile(b, nt);
+    double2* Hk = H + t.k * n * n;
+    const float2* Tk = T + t.k * n * n;
+    __syncthreads();                          // the last tile's mirror is written
+    for (int q = row0; q < 32; q += 8) {
+      const int i = t.i0 + lane, j = t.j0 + q;
+      if (i < n && j <= i) {
+        const size_t off = (size_t)j * n + i;
+        double2 h = Hk[off];
+        const float2 x = Tk[off];
+        h.x += (double)x.x;
+        h.y += (double)x.y;
+        Hk[off] = h;
+        tile[q][lane] = h;
+      }
+    }
+    __syncthreads();
+    for (int q = row0; q < 32; q += 8) {
+      const int i = t.i0 + q, j = t.j0 + lane;
+      if (i < n && j < i) Hk[(size_t)i * n + j] = make_double2(tile[lane][q].x, -tile[lane][q].y);
+    }
+  }
+}
+
+// H (FP64) := H + T (FP32), and the FP32 copy of the sum
+__global__ void add_f32_kernel(double* __restrict__ H, const float* __restrict__ T, float* __restrict__ copy32,
                                size_t n2) {
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n2;
        i += (size_t)gridDim.x * blockDim.x) {
-    const double v = base[i] + (double)add[i];
-    out[i] = v;
-    if (copy32) copy32[i] = (float)v;
+    const double v = H[i] + (double)T[i];
+    H[i] = v;
+    copy32[i] = (float)v;
   }
 }
-
-// Sh := I (the transformed pencil is standard)
-__global__ void set_identity_kernel(double* __restrict__ S, int n, size_t total) {
-  for (size_t idx = blockIdx.x * (size_t)blockDim.x + threadIdx.x; idx < total;
-       idx += (size_t)gridDim.x * blockDim.x) {
-    const size_t r = idx % ((size_t)n * n);
-    S[2 * idx] = ((int)(r % n) == (int)(r / n)) ? 1.0 : 0.0;
-    S[2 * idx + 1] = 0.0;
-  }
-}
-
 
 }  // namespace
 
-// Hh := (I+F)^H Hh (I+F), Sh := I, X := X (I+F) with F = -E/2 + 3E^2/8, E = Sh - I.
-// The products with the small F run as FP32-accurate tensor-core products
-// (olc_tcgemm.cu): their relative error times |F| ~ 1e-5 is far below FP64
-// needs.
-int loewdin(olc_context* ctx, int n, int nk, double* Hh, double* Sh, float* X) {
+// Hh := (I+F)^H Hh (I+F) and, where X != nullptr, X := X (I+F) with
+// F = -E/2 + 3E^2/8, E = Sh - I: the pencil is then standard.  The products
+// with the small F run as FP32-accurate tensor-core products (olc_tcgemm.cu):
+// their relative error times |F| ~ 1e-5 is far below FP64 needs.  E^2 and the
+// transformed Hh are Hermitian and form their lower tiles only; X matters to
+// the eigenvectors alone.
+int loewdin(olc_context* ctx, int n, int nk, double* Hh, const double* Sh, float* X) {
   cudaStream_t stream = ctx->stream;
   const size_t nn = (size_t)n * n, total = nn * nk;
   const long long s2 = 2 * (long long)nn;     // batch stride in floats
@@ -664,30 +726,33 @@ int loewdin(olc_context* ctx, int n, int nk, double* Hh, double* Sh, float* X) {
     StageScope scope(ctx, OLC_STAGE_REFINE, 1);
     loewdin_prep_kernel<<<grid_for(total), 256, 0, stream>>>(Hh, Sh, n, total, E, H32);
   }
-  auto gemm = [&](const float* A, bool conjA, const float* B, float beta, float* C) {
-    return tc::cgemm_f32(ctx, n, n, n, A, s2, n, conjA, B, s2, n, 1.f, beta, C, s2, n, nk, OLC_STAGE_REFINE);
+  auto gemm = [&](const float* A, bool conjA, const float* B, float beta, float* C, bool lower) {
+    return tc::cgemm_f32(ctx, n, n, n, A, s2, n, conjA, B, s2, n, 1.f, beta, C, s2, n, nk, OLC_STAGE_REFINE, lower);
   };
-  if ((st = gemm(E, false, E, 0.f, F))) return st;                 // F = E^2
+  const size_t nt = (n + 31) / 32;
+  const int tiles = (int)std::min<size_t>(nt * (nt + 1) / 2 * nk, 152 * 32);
+  if ((st = gemm(E, false, E, 0.f, F, true))) return st;           // F = E^2
   {
     StageScope scope(ctx, OLC_STAGE_REFINE, 1);
-    loewdin_f_kernel<<<grid_for(2 * total), 256, 0, stream>>>(E, F, 2 * total);
+    loewdin_f_kernel<<<tiles, 256, 0, stream>>>(reinterpret_cast<const float2*>(E), reinterpret_cast<float2*>(F), n,
+                                                nk);
   }
   // W = Hh + Hh F  (into Hh, FP32 copy into H32)
-  if ((st = gemm(H32, false, F, 0.f, T))) return st;
+  if ((st = gemm(H32, false, F, 0.f, T, false))) return st;
   {
     StageScope scope(ctx, OLC_STAGE_REFINE, 1);
-    add_f32_kernel<<<grid_for(2 * total), 256, 0, stream>>>(Hh, Hh, T, H32, 2 * total);
+    add_f32_kernel<<<grid_for(2 * total), 256, 0, stream>>>(Hh, T, H32, 2 * total);
   }
   // Hh' = W + F^H W
-  if ((st = gemm(F, true, H32, 0.f, T))) return st;
+  if ((st = gemm(F, true, H32, 0.f, T, true))) return st;
   {
-    StageScope scope(ctx, OLC_STAGE_REFINE, 2);
-    add_f32_kernel<<<grid_for(2 * total), 256, 0, stream>>>(Hh, Hh, T, nullptr, 2 * total);
-    set_identity_kernel<<<grid_for(total), 256, 0, stream>>>(Sh, n, total);
+    StageScope scope(ctx, OLC_STAGE_REFINE, 1);
+    add_hermitian_kernel<<<tiles, 256, 0, stream>>>(reinterpret_cast<double2*>(Hh), reinterpret_cast<float2*>(T), n,
+                                                    nk);
   }
   // X' = X + X F (the operand is split into BF16 pieces before the product
   // writes, so X may be both operand and output)
-  if ((st = gemm(X, false, F, 1.f, X))) return st;
+  if (X && (st = gemm(X, false, F, 1.f, X, false))) return st;
   cudaFreeAsync(E, stream);
   cudaFreeAsync(F, stream);
   cudaFreeAsync(H32, stream);
@@ -761,7 +826,8 @@ int solve_full_mixed(olc_context* ctx, const double* h, const double* s, int num
   // ---- 3. Loewdin transform: Sh = I + E  ->  (I+F)^H Hh (I+F), F = -E/2 + 3E^2/8
   // so that the pencil is standard; the products with the small F need only
   // FP32 (their relative error times |F| ~ 1e-5 is far below FP64 needs)
-  if ((st = loewdin(ctx, n, nk, Hh, Sh, X))) return st;
+  if ((st = loewdin(ctx, n, nk, Hh, Sh, vectors ? X : nullptr))) return st;
+  cudaFreeAsync(Sh, stream);
   // ---- 4. clusters and their exact solves -----------------------------------
   ClusterLists L{};
   L.cap = n * nk;                 // every cluster holds at least one state
@@ -844,7 +910,6 @@ int solve_full_mixed(olc_context* ctx, const double* h, const double* s, int num
   cudaFreeAsync(reach, stream);
   if (v_slot) cudaFreeAsync(v_slot, stream);
   cudaFreeAsync(Hh, stream);
-  cudaFreeAsync(Sh, stream);
   cudaFreeAsync(X, stream);
   if (st || !check) return st;
   return mixed_check_info(ctx);
