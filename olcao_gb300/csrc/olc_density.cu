@@ -16,8 +16,8 @@
 //    B = X_occ^H, zero-padded to the largest occupied count over k;
 //  * rho(k) = A B is one batched FP64-accurate split product on the tensor
 //    cores (olc_ozaki.cu, 53 bits per operand);
-//  * one HBM-bound pass reads every operator's upper triangle once against
-//    rho's and writes per-block partial traces, which a second kernel sums
+//  * one pass reads every operator's upper triangle once against both channels of
+//    rho, packs rho, and writes per-block partial traces, which a second kernel sums
 //    in a fixed order (bitwise reproducible from run to run).
 // The overlap comes from the prepared full S; NP, KE and V_j from the stored
 // packed terms, or, for a context prepared in the fused form, recomputed one
@@ -66,64 +66,74 @@ __global__ void gather_occupied_kernel(const double* __restrict__ X, int n, int 
   }
 }
 
-// spin = 2: (up, down) -> (up + down, up - down) over the upper triangles
-// (valeCharge.F90:307-313).
-__global__ void spin_sum_diff_kernel(double* __restrict__ r0, double* __restrict__ r1, int n, int nk) {
-  const size_t total = (size_t)nk * n * n;
-  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < total;
-       e += (size_t)gridDim.x * blockDim.x) {
-    const size_t m = e % ((size_t)n * n);
-    const int i = (int)(m / n), j = (int)(m % n);
-    if (j > i) continue;
-    const double ar = r0[2 * e], ai = r0[2 * e + 1], br = r1[2 * e], bi = r1[2 * e + 1];
-    r0[2 * e] = ar + br;
-    r0[2 * e + 1] = ai + bi;
-    r1[2 * e] = ar - br;
-    r1[2 * e + 1] = ai - bi;
+// A tile's share of the traces against the packed terms npk .. nt: two operators'
+// loads in flight; FULL: every row of the warp's tile holds elements.
+template <int NR, bool FULL>
+__device__ __forceinline__ void trace_terms(const double* __restrict__ terms, long long tstride, int npk, int nt,
+                                            size_t koff, const long long (&pr)[kTraceEpt],
+                                            const double (&wr)[NR][kTraceEpt], const double (&wi)[NR][kTraceEpt],
+                                            int rows, double* sacc) {
+  for (int t = npk; t < nt; t += 2) {
+    const bool two = t + 1 < nt;
+    const double2* t0 = reinterpret_cast<const double2*>(terms + (size_t)(t - npk) * tstride) + koff;
+    const double2* t1 = reinterpret_cast<const double2*>(terms + (size_t)(t + two - npk) * tstride) + koff;
+    double2 v0[kTraceEpt], v1[kTraceEpt];
+#pragma unroll
+    for (int e = 0; e < kTraceEpt; ++e)
+      if (FULL || e < rows) {
+        v0[e] = t0[pr[e]];
+        if (two) v1[e] = t1[pr[e]];
+      }
+#pragma unroll
+    for (int s = 0; s < NR; ++s) {
+      double a0 = 0.0, a1 = 0.0;
+#pragma unroll
+      for (int e = 0; e < kTraceEpt; ++e)
+        if (FULL || e < rows) {
+          a0 = fma(v0[e].x, wr[s][e], fma(v0[e].y, wi[s][e], a0));   // two instructions, not three
+          if (two) a1 = fma(v1[e].x, wr[s][e], fma(v1[e].y, wi[s][e], a1));
+        }
+      sacc[(s * nt + t) * kTraceThreads] += a0;
+      if (two) sacc[(s * nt + t + 1) * kTraceThreads] += a1;
+    }
   }
 }
 
-// packMatrix of every k (matrixSubs.F90:400-425): full [nk][n][n] -> packed
-// [nk][plen][2], index j + i(i+1)/2 for row j <= column i.
-__global__ void pack_rho_kernel(const double* __restrict__ full, int n, int nk, double* __restrict__ packed) {
-  const size_t plen = (size_t)n * (n + 1) / 2, total = plen * nk;
-  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < total;
-       e += (size_t)gridDim.x * blockDim.x) {
-    const int k = (int)(e / plen);
-    const size_t r = e % plen;
-    int i = (int)((sqrt(8.0 * (double)r + 1.0) - 1.0) * 0.5);
-    while ((size_t)i * (i + 1) / 2 > r) --i;
-    while ((size_t)(i + 1) * (i + 2) / 2 <= r) ++i;
-    const int j = (int)(r - (size_t)i * (i + 1) / 2);
-    const size_t off = (size_t)k * n * n + (size_t)i * n + j;
-    packed[2 * e] = full[2 * off];
-    packed[2 * e + 1] = full[2 * off + 1];
-  }
-}
-
-// Element-wise traces of rho against nt operators.  Operator 0 is the full
-// S [nk][n][n] when sfull != nullptr; the others are packed terms
-// [nt'][nk][plen][2] (term stride tstride doubles).  Block (b, k) walks tiles
-// b, b + gridDim.x, ... of k's packed index range.  Every thread keeps one
-// running sum per operator in shared memory (sacc[t][thread]), so the inner
-// loop has no cross-thread traffic; the block reduces them once at the end
-// and writes partial[(k * gridDim.x + b) * nt + t].  Each pass over a tile
-// has the loads of two operators in flight.
+// Element-wise traces of NR density matrices against nt operators.  rho holds
+// the spin channels (stride rstride doubles); for NR = 2 the traces are those
+// of up + down and up - down (valeCharge.F90:307-313), formed in registers.
+// Operator 0 is the full S [nk][n][n] when sfull != nullptr; the others are
+// packed terms [nt'][nk][plen][2] (term stride tstride doubles).  Block (b, k)
+// walks tiles b, b + gridDim.x, ... of k's packed index range.  Every thread
+// keeps one running sum per matrix and operator in shared memory
+// (sacc[s * nt + t][thread]), so the inner loop has no cross-thread traffic; the
+// block reduces them once at the end and writes
+// partial[((k * gridDim.x + b) * NR + s) * nt + t].  Each pass over a tile
+// has the loads of two operators in flight.  packed != nullptr receives the
+// matrices as packMatrix orders them (matrixSubs.F90:400-425): [NR][nk][plen][2],
+// index j + i(i+1)/2 for row j <= column i.
+// Bound by the FP64 pipe, two multiply-adds per element, operator and matrix;
+// both spin channels share one read of the operators.  A pass per channel with
+// the sums, differences and packing in kernels of their own took 3.1 ms for 19
+// operators of order 832 at 27 k-points, this form 1.6 ms.
+template <int NR>
 __global__ void __launch_bounds__(kTraceThreads) trace_kernel(
-    const double* __restrict__ rho, const double* __restrict__ sfull, const double* __restrict__ terms,
-    long long tstride, int nt, int n, long long plen, double* __restrict__ partial) {
-  extern __shared__ double sacc[];           // [nt][kTraceThreads]
+    const double* __restrict__ rho, size_t rstride, const double* __restrict__ sfull, const double* __restrict__ terms,
+    long long tstride, int nt, int n, long long plen, double* __restrict__ partial, double* __restrict__ packed) {
+  extern __shared__ double sacc[];           // [NR][nt][kTraceThreads]
   const int k = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  for (int t = 0; t < nt; ++t) sacc[t * kTraceThreads + tid] = 0.0;
+  for (int t = 0; t < NR * nt; ++t) sacc[t * kTraceThreads + tid] = 0.0;
   const size_t nn = (size_t)n * n;
   const double2* rk = reinterpret_cast<const double2*>(rho) + (size_t)k * nn;
   const double2* sk = sfull ? reinterpret_cast<const double2*>(sfull) + (size_t)k * nn : nullptr;
   const int npk = sfull ? 1 : 0;
   const long long tile = (long long)kTraceThreads * kTraceEpt;
   for (long long base = (long long)blockIdx.x * tile; base < plen; base += (long long)gridDim.x * tile) {
-    double wr[kTraceEpt], wi[kTraceEpt];
-    size_t foff[kTraceEpt];
+    double wr[NR][kTraceEpt], wi[NR][kTraceEpt];
     long long pr[kTraceEpt];
+    double a[NR];
+#pragma unroll
+    for (int s = 0; s < NR; ++s) a[s] = 0.0;
 #pragma unroll
     for (int e = 0; e < kTraceEpt; ++e) {
       const long long r = base + (long long)e * kTraceThreads + tid;
@@ -132,79 +142,71 @@ __global__ void __launch_bounds__(kTraceThreads) trace_kernel(
       while ((long long)i * (i + 1) / 2 > pr[e]) --i;
       while ((long long)(i + 1) * (i + 2) / 2 <= pr[e]) ++i;
       const int j = (int)(pr[e] - (long long)i * (i + 1) / 2);
-      foff[e] = (size_t)i * n + j;
-      const double2 x = rk[foff[e]];
+      const size_t foff = (size_t)i * n + j;
+      double2 x[NR];
+#pragma unroll
+      for (int s = 0; s < NR; ++s) x[s] = rk[s * (rstride / 2) + foff];
+      if (NR == 2) {
+        const double2 u = x[0], d = x[NR - 1];
+        x[0] = make_double2(u.x + d.x, u.y + d.y);
+        x[NR - 1] = make_double2(u.x - d.x, u.y - d.y);
+      }
+      if (packed && r < plen) {
+#pragma unroll
+        for (int s = 0; s < NR; ++s) {
+          double* o = packed + 2 * (((size_t)s * gridDim.y + k) * plen + r);   // the caller's: any 8-byte address
+          o[0] = x[s].x;
+          o[1] = x[s].y;
+        }
+      }
       // the diagonal counts once and only its real part; off-diagonal
       // elements stand for themselves and their mirror image
       const double g = r < plen ? (i == j ? 1.0 : 2.0) : 0.0;
-      wr[e] = g * x.x;
-      wi[e] = (i == j) ? 0.0 : g * x.y;
+      const double2 v = npk ? sk[foff] : make_double2(0.0, 0.0);
+#pragma unroll
+      for (int s = 0; s < NR; ++s) {
+        wr[s][e] = g * x[s].x;
+        wi[s][e] = (i == j) ? 0.0 : g * x[s].y;
+        if (npk) a[s] = fma(v.x, wr[s][e], fma(v.y, wi[s][e], a[s]));
+      }
     }
-    int t = 0;
     if (npk) {
-      double a = 0.0;
 #pragma unroll
-      for (int e = 0; e < kTraceEpt; ++e) {
-        const double2 v = sk[foff[e]];
-        a += v.x * wr[e] + v.y * wi[e];
-      }
-      sacc[tid] += a;
-      t = 1;
+      for (int s = 0; s < NR; ++s) sacc[s * nt * kTraceThreads + tid] += a[s];
     }
-    for (; t + 1 < nt; t += 2) {
-      const double2* t0 = reinterpret_cast<const double2*>(terms + (size_t)(t - npk) * tstride) + (size_t)k * plen;
-      const double2* t1 = reinterpret_cast<const double2*>(terms + (size_t)(t + 1 - npk) * tstride) + (size_t)k * plen;
-      double2 v0[kTraceEpt], v1[kTraceEpt];
-#pragma unroll
-      for (int e = 0; e < kTraceEpt; ++e) {
-        v0[e] = t0[pr[e]];
-        v1[e] = t1[pr[e]];
-      }
-      double a0 = 0.0, a1 = 0.0;
-#pragma unroll
-      for (int e = 0; e < kTraceEpt; ++e) {
-        a0 += v0[e].x * wr[e] + v0[e].y * wi[e];
-        a1 += v1[e].x * wr[e] + v1[e].y * wi[e];
-      }
-      sacc[t * kTraceThreads + tid] += a0;
-      sacc[(t + 1) * kTraceThreads + tid] += a1;
-    }
-    if (t < nt) {
-      const double2* t0 = reinterpret_cast<const double2*>(terms + (size_t)(t - npk) * tstride) + (size_t)k * plen;
-      double a0 = 0.0;
-#pragma unroll
-      for (int e = 0; e < kTraceEpt; ++e) {
-        const double2 v = t0[pr[e]];
-        a0 += v.x * wr[e] + v.y * wi[e];
-      }
-      sacc[t * kTraceThreads + tid] += a0;
-    }
+    // rows of this warp that hold elements: all but in the last tile
+    const long long left = plen - base - (tid & ~31);
+    const int rows = left <= 0 ? 0 : (int)min((left + kTraceThreads - 1) / kTraceThreads, (long long)kTraceEpt);
+    if (rows == kTraceEpt)
+      trace_terms<NR, true>(terms, tstride, npk, nt, (size_t)k * plen, pr, wr, wi, rows, sacc + tid);
+    else if (rows > 0)
+      trace_terms<NR, false>(terms, tstride, npk, nt, (size_t)k * plen, pr, wr, wi, rows, sacc + tid);
   }
   __syncthreads();
-  for (int t = warp; t < nt; t += kTraceThreads / 32) {
+  for (int t = warp; t < NR * nt; t += kTraceThreads / 32) {
     double a = 0.0;
     for (int q = lane; q < kTraceThreads; q += 32) a += sacc[t * kTraceThreads + q];
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) a += __shfl_down_sync(0xffffffffu, a, o);
-    if (lane == 0) partial[((size_t)k * gridDim.x + blockIdx.x) * nt + t] = a;
+    if (lane == 0) partial[((size_t)k * gridDim.x + blockIdx.x) * NR * nt + t] = a;
   }
 }
 
-// out[t] = sum over the np partial rows of partial[row * nt + t], in a fixed
-// order: one block per t.
-__global__ void reduce_partials_kernel(const double* __restrict__ partial, int np, int nt,
+// out[s * ostride + t] = sum over the np partial rows of
+// partial[(row * gridDim.y + s) * nt + t], in a fixed order: one block per (t, s).
+__global__ void reduce_partials_kernel(const double* __restrict__ partial, int np, int nt, int ostride,
                                        double* __restrict__ out) {
-  __shared__ double s[256];
-  const int t = blockIdx.x;
+  __shared__ double sum[256];
+  const int t = blockIdx.x, s = blockIdx.y;
   double a = 0.0;
-  for (int q = threadIdx.x; q < np; q += blockDim.x) a += partial[(size_t)q * nt + t];
-  s[threadIdx.x] = a;
+  for (int q = threadIdx.x; q < np; q += blockDim.x) a += partial[((size_t)q * gridDim.y + s) * nt + t];
+  sum[threadIdx.x] = a;
   __syncthreads();
   for (int h = blockDim.x / 2; h > 0; h >>= 1) {
-    if ((int)threadIdx.x < h) s[threadIdx.x] += s[threadIdx.x + h];
+    if ((int)threadIdx.x < h) sum[threadIdx.x] += sum[threadIdx.x + h];
     __syncthreads();
   }
-  if (threadIdx.x == 0) out[t] = s[0];
+  if (threadIdx.x == 0) out[s * ostride + t] = sum[0];
 }
 
 struct Scratch {
@@ -224,22 +226,37 @@ struct Scratch {
   }
 };
 
-// Traces of rho (all k) against nt operators into out[nt] (device), in
-// chunks of at most kTraceChunk operators (per-thread accumulators of one
-// chunk fill 48 KB of shared memory).
-int launch_traces(olc_context* ctx, const double* rho, const double* sfull, const double* terms,
-                  long long tstride, int nt, double* partial, int bx, double* out) {
+// Resident blocks of a full chunk's trace kernel on the whole device.
+int trace_blocks(int spin) {
+  int dev = 0, sms = 0, per = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const size_t smem = sizeof(double) * kTraceThreads * kTraceChunk * spin;
+  const auto kern = spin == 2 ? trace_kernel<2> : trace_kernel<1>;
+  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, kTraceThreads, smem) != cudaSuccess) per = 1;
+  return std::max(1, per) * sms;
+}
+
+// Traces of rho (all k, `spin` channels of stride rstride) against nt operators
+// into out[s * ostride + t] (device), in chunks of at most kTraceChunk operators
+// (per-thread accumulators of one chunk and channel fill 48 KB of shared
+// memory).  packed: see trace_kernel.
+int launch_traces(olc_context* ctx, const double* rho, int spin, const double* sfull, const double* terms,
+                  long long tstride, int nt, double* partial, int bx, double* out, int ostride, double* packed) {
   const int n = ctx->dims.vale_dim, nk = ctx->dims.num_kpoints;
   const long long plen = ctx->dims.packed_len;
+  const size_t rstride = 2 * (size_t)n * n * nk;
+  const auto kern = spin == 2 ? trace_kernel<2> : trace_kernel<1>;
   StageScope scope(ctx, OLC_STAGE_DENSITY, 0);
   for (int t0 = 0; t0 < nt; t0 += kTraceChunk) {
     const int c = std::min(kTraceChunk, nt - t0);
     const bool with_s = sfull && t0 == 0;
     const double* tp = terms ? terms + (size_t)(t0 - (sfull && t0 > 0 ? 1 : 0)) * tstride : nullptr;
-    const size_t smem = sizeof(double) * kTraceThreads * c;
-    trace_kernel<<<dim3(bx, nk), kTraceThreads, smem, ctx->stream>>>(rho, with_s ? sfull : nullptr, tp, tstride, c,
-                                                                      n, plen, partial);
-    reduce_partials_kernel<<<c, 256, 0, ctx->stream>>>(partial, bx * nk, c, out + t0);
+    const size_t smem = sizeof(double) * kTraceThreads * c * spin;
+    kern<<<dim3(bx, nk), kTraceThreads, smem, ctx->stream>>>(rho, rstride, with_s ? sfull : nullptr, tp, tstride, c, n,
+                                                              plen, partial, t0 == 0 ? packed : nullptr);
+    reduce_partials_kernel<<<dim3(c, spin), 256, 0, ctx->stream>>>(partial, bx * nk, c, ostride, out + t0);
     scope.add_launches(2);
   }
   return cuda_check(cudaGetLastError(), "trace kernels");
@@ -327,38 +344,24 @@ int make_valence_rho(olc_context* ctx, int num_states, int spin, const double* o
                                           true)))
       return rc;
   }
-  double* rho1 = rho + 2 * nn * nk;
-  if (spin == 2) {
-    StageScope scope(ctx, OLC_STAGE_DENSITY);
-    spin_sum_diff_kernel<<<grid_of(nn * nk), 256, 0, st>>>(rho, rho1, n, nk);
-  }
-  if (rho_packed) {
-    StageScope scope(ctx, OLC_STAGE_DENSITY, spin);
-    const size_t pl2 = 2 * (size_t)ctx->dims.packed_len * nk;
-    for (int s = 0; s < spin; ++s)
-      pack_rho_kernel<<<grid_of(pl2 / 2), 256, 0, st>>>(rho + 2 * (size_t)s * nn * nk, n, nk, rho_packed + s * pl2);
-  }
-
   // element-wise traces: S from the prepared full overlap, then NP, KE, V_j
   const long long plen = ctx->dims.packed_len;
   const long long tiles = (plen + (long long)kTraceThreads * kTraceEpt - 1) / ((long long)kTraceThreads * kTraceEpt);
-  const int bx = (int)std::max<long long>(1, std::min<long long>(tiles, (152LL * 8 + nk - 1) / nk));
-  if ((rc = sc.get(&partial, sizeof(double) * (size_t)bx * nk * nt, "malloc partial traces"))) return rc;
+  // one wave of the trace kernel's blocks over all k
+  const int bx = (int)std::max<long long>(1, std::min<long long>(tiles, (long long)trace_blocks(spin) / nk));
+  if ((rc = sc.get(&partial, sizeof(double) * (size_t)bx * nk * nt * spin, "malloc partial traces"))) return rc;
   const long long tstride = 2 * plen * nk;
   if (ctx->prep_form == OLC_FORM_STORED && ctx->d_terms) {
     // d_terms holds NP, KE, (MV,) V_j in the trace order of the reference
-    for (int s = 0; s < spin; ++s)
-      if ((rc = launch_traces(ctx, rho + 2 * (size_t)s * nn * nk, ctx->d_chol, ctx->d_terms, tstride, nt, partial,
-                              bx, dtr + (size_t)s * nt))) return rc;
+    if ((rc = launch_traces(ctx, rho, spin, ctx->d_chol, ctx->d_terms, tstride, nt, partial, bx, dtr, nt, rho_packed)))
+      return rc;
   } else {
     // fused form: no operator is kept apart, so each is recomputed,
     // orthogonalised and packed once into scratch (as olc_scf_prepare's
     // stored form builds them) and traced for every spin channel
     double* tmp = nullptr;
     if ((rc = sc.get(&tmp, 8 * (size_t)tstride, "malloc packed operator"))) return rc;
-    for (int s = 0; s < spin; ++s)
-      if ((rc = launch_traces(ctx, rho + 2 * (size_t)s * nn * nk, ctx->d_chol, nullptr, 0, 1, partial, bx,
-                              dtr + (size_t)s * nt))) return rc;
+    if ((rc = launch_traces(ctx, rho, spin, ctx->d_chol, nullptr, 0, 1, partial, bx, dtr, nt, rho_packed))) return rc;
     const int ops[3] = {OLC_OP_NUCLEAR, OLC_OP_KINETIC, OLC_OP_MASSVEL};
     for (int t = 0; t < nfix + pd; ++t) {
       const int op = t < nfix ? ops[t] : OLC_OP_ELECPOT;
@@ -366,9 +369,8 @@ int make_valence_rho(olc_context* ctx, int num_states, int spin, const double* o
       if ((rc = run_contract_bloch(ctx, ctx->d_work_vv, ctx->d_work_cv, ctx->d_work_cc))) return rc;
       if ((rc = ortho_pack(ctx, false, ctx->d_work_vv, ctx->d_work_cv, ctx->d_work_cc, ctx->d_scv, tmp, nullptr)))
         return rc;
-      for (int s = 0; s < spin; ++s)
-        if ((rc = launch_traces(ctx, rho + 2 * (size_t)s * nn * nk, nullptr, tmp, tstride, 1, partial, bx,
-                                dtr + (size_t)s * nt + 1 + t))) return rc;
+      if ((rc = launch_traces(ctx, rho, spin, nullptr, tmp, tstride, 1, partial, bx, dtr + 1 + t, nt, nullptr)))
+        return rc;
     }
   }
   if ((rc = cuda_check(cudaMemcpyAsync(traces, dtr, sizeof(double) * nt * spin, cudaMemcpyDeviceToHost, st),
