@@ -59,12 +59,8 @@ namespace {
 constexpr int BM = 128;            // rows per tile (TMEM lanes)
 constexpr int BK = 64;             // K per stage: 64 BF16 = one 128-byte swizzle row
 constexpr int MAX_SLOTS = 8;       // plane slots per operand
-// epilogue warps: the fixed mode's 64-bit sums want registers, the f32 mode's
-// drains want loads in flight
-template <int MODE>
-constexpr int epi_warps() { return MODE == 0 ? 8 : 16; }
-template <int MODE>
-constexpr int num_threads() { return (epi_warps<MODE>() + 2) * 32; }
+constexpr int kEpiWarps = 16;      // loads in flight for the drains; 96 registers hold 32 64-bit sums
+constexpr int kThreads = (kEpiWarps + 2) * 32;
 // accumulators: four of 128 columns (fixed mode), two of 256 (f32 mode)
 template <int MODE>
 constexpr int num_acc() { return MODE == 0 ? 4 : 2; }
@@ -160,6 +156,19 @@ __device__ __forceinline__ void tmem_ld16(uint32_t ta, uint32_t (&r)[16]) {
         "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
       : "r"(ta));
 }
+__device__ __forceinline__ void tmem_ld8(uint32_t ta, uint32_t (&r)[8]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+               : "r"(ta));
+}
+// Waits for every load issued so far; r, the values about to be used, passes
+// through so that no use of it moves ahead of the wait.
+__device__ __forceinline__ void tmem_ld_wait(uint32_t (&r)[8]) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7])
+               :
+               : "memory");
+}
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
 // Tile of a CTA: grouped raster (GM row tiles at a time) so that the CTAs in
@@ -187,13 +196,14 @@ inline int smem_total(int mode, int slots_a, int slots_b) {
 // ---------------------------------------------------------------------------
 // the kernel
 // ---------------------------------------------------------------------------
-// What bounds it: in the fixed mode the drains (a 128 x 128 accumulator through
-// tcgen05.ld, exact conversion and 64-bit multiply-adds) and the issue of the
-// MMAs, 79 clocks each at N = 128, run about level; in the f32 mode the copies'
-// latency at the K-steps' ends.  Measured: FP64-accurate product of order 1248
-// 1025 -> 850 us, FP32-accurate 78 -> 83 us (one partial wave), 64 products of
-// order 832 with 17 digit pairs 7.3 -> 6.1 ms each, the FP32-accurate products
-// of a pass over 8 matrices of order 2808 72 -> 55 ms.
+// What bounds it: in the fixed mode the copies from L2 and the MMAs one after the
+// other: a K-block's 14 tiles of 16 KB fill shared memory and are all in use
+// for half of its pairs, the copies run at the 5.4 TB/s that all SMs together
+// reach, and what is left of the 34 pairs hides about a third of them.  In the
+// f32 mode the copies' latency at the K-steps' ends.  Measured: FP64-accurate
+// product of order 1248 1025 -> 818 us, FP32-accurate 78 -> 83 us (one partial
+// wave); a mixed pass over 64 matrices of order 832: FP64-accurate products
+// 22.7 -> 19 ms, FP32-accurate ones (as then formed) 18.5 -> 14.2 ms.
 // MODE 0 (fixed): BN = 128, four accumulators of 128 columns, int64 drains,
 //   FP64 complex output.  Epilogue warp w owns TMEM lanes 32 (w % 4) .. +31
 //   and columns 32 (w / 4) .. +31 of the tile (16 complex columns).
@@ -201,15 +211,15 @@ inline int smem_total(int mode, int slots_a, int slots_b) {
 //   alpha, beta; warp w owns columns 64 (w / 4) .. +63 (32 complex).
 
 template <int MODE>
-__global__ void __launch_bounds__(num_threads<MODE>(), 1)
+__global__ void __launch_bounds__(kThreads, 1)
     tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                    const __grid_constant__ TcParams p) {
   constexpr int BN = MODE == 0 ? 128 : 256;
   constexpr int NACC = num_acc<MODE>();
   constexpr uint32_t IDESC = idesc_bf16(BM, BN);
   constexpr int TB = tile_bytes_b<MODE>();
-  constexpr int PRODUCER_WARP = epi_warps<MODE>(), MMA_WARP = PRODUCER_WARP + 1;
-  constexpr int CW = 4 * BN / epi_warps<MODE>();      // columns of an epilogue warp
+  constexpr int PRODUCER_WARP = kEpiWarps, MMA_WARP = PRODUCER_WARP + 1;
+  constexpr int CW = 4 * BN / kEpiWarps;      // columns of an epilogue warp
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   uint8_t* smem = smem_raw + (((raw + 1023u) & ~1023u) - raw);
@@ -259,7 +269,7 @@ __global__ void __launch_bounds__(num_threads<MODE>(), 1)
     }
     for (int s = 0; s < NACC; ++s) {
       mbar_init(&accfull[s], 1);
-      mbar_init(&accempty[s], epi_warps<MODE>());
+      mbar_init(&accempty[s], kEpiWarps);
     }
     *cta_err = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -279,47 +289,53 @@ __global__ void __launch_bounds__(num_threads<MODE>(), 1)
     if (lane == 0) {
       asm volatile("prefetch.tensormap [%0];" ::"l"(&tmA) : "memory");
       asm volatile("prefetch.tensormap [%0];" ::"l"(&tmB) : "memory");
-      int sa = 0, sb = 0;               // next slots; their wrap-around parities
-      uint32_t pha = 0, phb = 0;
-      int na = 0, nb = 0;               // copies issued
+      int basea = 0, baseb = 0;         // slots of this K-step's tile 0
+      uint32_t pha = 0, phb = 0;        // their wrap-around parities
       const int span = p.kspan - 1;     // 0 or 1
+      uint32_t seen[2] = {0u, 0u}, par[2] = {0u, 0u};   // slots in use and the parities of their last copies
       bool ok = true;
       for (int kb = 0; kb < p.kblocks && ok; ++kb) {
         if (!kb_needed(kb)) continue;
-        for (int i = 0; i < p.npairs; ++i) {
-          const TcPair pr = p.pairs[i];
-          if (pr.flags & kPairFirstA) {
-            if (!mbar_wait(&emptyA[sa], pha ^ 1u, cta_err, p.err, 1)) { ok = false; break; }
-            mbar_expect_tx(&fullA[sa], (uint32_t)kTileBytesA);
-            const int pl = MODE == 0 ? pr.pa >> span : pr.pa, k0 = MODE == 0 ? (kb << span) + (pr.pa & span) : kb;
-            tma_load_3d(sA + sa * kTileBytesA, &tmA, &fullA[sa], k0 * BK, m0, b * p.planes_a + pl);
-            ++na;
-            if (++sa == p.slots_a) { sa = 0; pha ^= 1u; }
-          }
-          if (pr.flags & kPairFirstB) {
-            if (!mbar_wait(&emptyB[sb], phb ^ 1u, cta_err, p.err, 1)) { ok = false; break; }
-            mbar_expect_tx(&fullB[sb], (uint32_t)TB);
+        for (int i = 0; i < p.nload; ++i) {
+          const int ld = p.load[i];
+          if (ld >= 0) {
+            int s = basea + ld;
+            uint32_t ph = pha;
+            while (s >= p.slots_a) { s -= p.slots_a; ph ^= 1u; }
+            if (!mbar_wait(&emptyA[s], ph ^ 1u, cta_err, p.err, 1)) { ok = false; break; }
+            mbar_expect_tx(&fullA[s], (uint32_t)kTileBytesA);
+            const int pl = MODE == 0 ? ld >> span : ld, k0 = MODE == 0 ? (kb << span) + (ld & span) : kb;
+            tma_load_3d(sA + s * kTileBytesA, &tmA, &fullA[s], k0 * BK, m0, b * p.planes_a + pl);
+            seen[0] |= 1u << s;
+            par[0] = (par[0] & ~(1u << s)) | (ph << s);
+          } else {
+            const int t = -1 - ld;
+            int s = baseb + t;
+            uint32_t ph = phb;
+            while (s >= p.slots_b) { s -= p.slots_b; ph ^= 1u; }
+            if (!mbar_wait(&emptyB[s], ph ^ 1u, cta_err, p.err, 1)) { ok = false; break; }
+            mbar_expect_tx(&fullB[s], (uint32_t)TB);
             // f32 mode: B's planes from the last to the first
-            const int pl = MODE == 0 ? pr.pb >> span : p.planes_b - 1 - pr.pb;
-            const int k0 = MODE == 0 ? (kb << span) + (pr.pb & span) : kb;
-            tma_load_3d(sB + sb * TB, &tmB, &fullB[sb], k0 * BK, n0, b * p.planes_b + pl);
-            ++nb;
-            if (++sb == p.slots_b) { sb = 0; phb ^= 1u; }
+            const int pl = MODE == 0 ? t >> span : p.planes_b - 1 - t, k0 = MODE == 0 ? (kb << span) + (t & span) : kb;
+            tma_load_3d(sB + s * TB, &tmB, &fullB[s], k0 * BK, n0, b * p.planes_b + pl);
+            seen[1] |= 1u << s;
+            par[1] = (par[1] & ~(1u << s)) | (ph << s);
           }
         }
+        basea += p.planes_a * p.kspan;
+        while (basea >= p.slots_a) { basea -= p.slots_a; pha ^= 1u; }
+        baseb += p.planes_b * p.kspan;
+        while (baseb >= p.slots_b) { baseb -= p.slots_b; phb ^= 1u; }
       }
       if (!ok) {
         // wait (bounded) for the copies still in flight before the CTA exits
-        auto settle = [&](uint64_t* full, int slots, int s, uint32_t ph, int issued) {
-          for (int q = 0; q < slots && q < issued; ++q) {
-            if (--s < 0) { s = slots - 1; ph ^= 1u; }
-            const unsigned long long t0 = now_ns();
-            while (!mbar_try(&full[s], ph) && (long long)(now_ns() - t0) < kWaitNs) {
-            }
+        for (int s = 0; s < 2 * MAX_SLOTS; ++s) {
+          const int o = s / MAX_SLOTS, q = s % MAX_SLOTS;
+          if (!(seen[o] >> q & 1u)) continue;
+          const unsigned long long t0 = now_ns();
+          while (!mbar_try(o ? &fullB[q] : &fullA[q], par[o] >> q & 1u) && (long long)(now_ns() - t0) < kWaitNs) {
           }
-        };
-        settle(fullA, p.slots_a, sa, pha, na);
-        settle(fullB, p.slots_b, sb, phb, nb);
+        }
       }
     }
   } else if (warp == MMA_WARP) {
@@ -332,37 +348,43 @@ __global__ void __launch_bounds__(num_threads<MODE>(), 1)
     bool ok = true;
     int buf = 0;                        // accumulator of the current group and its wrap-around parity
     uint32_t phacc = 1;
+    TcPair pr = p.pairs[0];             // the next pair is read while this one is issued
     for (int kb = 0; kb < p.kblocks && ok; ++kb) {
       if (!kb_needed(kb)) continue;
       for (int i = 0; i < p.npairs; ++i) {
-        const TcPair pr = p.pairs[i];
-        // tiles enter the rings in the order of their first use, 0, 1, ...
+        const int flags = pr.flags;
         int sa = basea + pr.pa, sb = baseb + pr.pb;
+        pr = p.pairs[i + 1 < p.npairs ? i + 1 : 0];
         uint32_t fa = pha, fb = phb;
-        while (sa >= p.slots_a) { sa -= p.slots_a; fa ^= 1u; }
-        while (sb >= p.slots_b) { sb -= p.slots_b; fb ^= 1u; }
-        const bool start = (pr.flags & kPairStart) != 0;
-        if (start) ok = mbar_wait(&accempty[buf], phacc, cta_err, p.err, 2);
-        if (ok && (pr.flags & kPairFirstA)) ok = mbar_wait(&fullA[sa], fa, cta_err, p.err, 3);
-        if (ok && (pr.flags & kPairFirstB)) ok = mbar_wait(&fullB[sb], fb, cta_err, p.err, 3);
-        if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
-        tc_fence_after();
+#pragma unroll
+        for (int w = 0; w < 2; ++w) {   // a step has fewer tiles than two turns of the ring
+          if (sa >= p.slots_a) { sa -= p.slots_a; fa ^= 1u; }
+          if (sb >= p.slots_b) { sb -= p.slots_b; fb ^= 1u; }
+        }
+        if (flags & (kPairStart | kPairFirstA | kPairFirstB)) {
+          if (flags & kPairStart) ok = mbar_wait(&accempty[buf], phacc, cta_err, p.err, 2);
+          if (ok && (flags & kPairFirstA)) ok = mbar_wait(&fullA[sa], fa, cta_err, p.err, 3);
+          if (ok && (flags & kPairFirstB)) ok = mbar_wait(&fullB[sb], fb, cta_err, p.err, 3);
+          if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
+          tc_fence_after();
+        }
         const uint32_t dt = tmem + (uint32_t)(buf * BN);
         const uint32_t al = a_lo + sa * (kTileBytesA >> 4), bl = b_lo + sb * (TB >> 4);
         if (leader) {
+          umma(dt, sdesc(al), sdesc(bl), IDESC, (flags & kPairStart) ? 0u : 1u);
 #pragma unroll
-          for (int k = 0; k < BK / 16; ++k)
+          for (int k = 1; k < BK / 16; ++k)
             // +32 bytes of K per instruction: +2 in the descriptor's address field
-            umma(dt, sdesc(al + 2 * k), sdesc(bl + 2 * k), IDESC, (start && k == 0) ? 0u : 1u);
-          if (pr.flags & kPairLastA) umma_commit(&emptyA[sa]);
-          if (pr.flags & kPairLastB) umma_commit(&emptyB[sb]);
-          if (pr.flags & kPairEnd) umma_commit(&accfull[buf]);
+            umma(dt, sdesc(al + 2 * k), sdesc(bl + 2 * k), IDESC, 1u);
+          if (flags & kPairLastA) umma_commit(&emptyA[sa]);
+          if (flags & kPairLastB) umma_commit(&emptyB[sb]);
+          if (flags & kPairEnd) umma_commit(&accfull[buf]);
         }
-        __syncwarp();
-        if (pr.flags & kPairEnd) {
+        if (flags & kPairEnd) {
           if (++buf == NACC) { buf = 0; phacc ^= 1u; }
         }
       }
+      __syncwarp();
       basea += p.planes_a * p.kspan;
       while (basea >= p.slots_a) { basea -= p.slots_a; pha ^= 1u; }
       baseb += p.planes_b * p.kspan;
@@ -387,35 +409,37 @@ __global__ void __launch_bounds__(num_threads<MODE>(), 1)
           if (!ok) break;
           tc_fence_after();
           const int sh = p.shift[i];
+          const uint32_t col = lane_addr + (uint32_t)(buf * BN + CW * h);
+          const auto drain = [&](auto add) {
+            // the next eight columns are under way while the last are added
+            uint32_t rr[2][8];
+            tmem_ld8(col, rr[0]);
 #pragma unroll
-          for (int part = 0; part < CW / 16; ++part) {
-            uint32_t r[16];
-            tmem_ld16(lane_addr + (uint32_t)(buf * BN + CW * h + 16 * part), r);
-            tmem_ld_wait();
-            if (part == CW / 16 - 1) {
-              tc_fence_before();
-              __syncwarp();
-              if (lane == 0) mbar_arrive(&accempty[buf]);
+            for (int part = 0; part < CW / 8; ++part) {
+              tmem_ld_wait(rr[part & 1]);
+              if (part < CW / 8 - 1) {
+                tmem_ld8(col + 8 * (part + 1), rr[(part + 1) & 1]);
+              } else {
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&accempty[buf]);
+              }
+#pragma unroll
+              for (int j = 0; j < 8; ++j) add(acc[8 * part + j], __float2int_rn(__uint_as_float(rr[part & 1][j])));
             }
-            if (sh > 30) {
-#pragma unroll
-              for (int j = 0; j < 16; ++j)
-                acc[16 * part + j] += (long long)__float2int_rn(__uint_as_float(r[j])) << sh;
-            } else if (sh >= 0) {
-              // one 32 x 32 + 64-bit multiply-add per sum
-              const int mul = 1 << sh;
-#pragma unroll
-              for (int j = 0; j < 16; ++j)
-                acc[16 * part + j] += (long long)__float2int_rn(__uint_as_float(r[j])) * mul;
-            } else {
-              // low-order digit groups: rounded to the accumulator's unit (a
-              // plain arithmetic shift would floor, a bias of half a unit per
-              // drain that adds up over long K)
-              const int half = 1 << (-sh - 1);
-#pragma unroll
-              for (int j = 0; j < 16; ++j)
-                acc[16 * part + j] += (__float2int_rn(__uint_as_float(r[j])) + half) >> (-sh);
-            }
+          };
+          if (sh > 30) {
+            drain([sh](long long& x, int v) { x += (long long)v << sh; });
+          } else if (sh >= 0) {
+            // one 32 x 32 + 64-bit multiply-add per sum
+            const int mul = 1 << sh;
+            drain([mul](long long& x, int v) { x += (long long)v * mul; });
+          } else {
+            // low-order digit groups: rounded to the accumulator's unit (a
+            // plain arithmetic shift would floor, a bias of half a unit per
+            // drain that adds up over long K)
+            const int half = 1 << (-sh - 1);
+            drain([sh, half](long long& x, int v) { x += (v + half) >> (-sh); });
           }
         }
       }
@@ -774,11 +798,12 @@ int make_map(CUtensorMap* map, const void* base, size_t Kp, size_t rows, size_t 
 int* g_err = nullptr;   // device error word shared by the launches of this process
 std::mutex g_err_mu;
 
-// First / last uses of the tiles, and the tile slots.  The slots cover what a
-// K-step keeps live plus what is staged ahead, 224 KB in all: fixed mode 14 of
-// 16 KB (7 + 7 digits in one K-block: all live at once; 3 + 6 digits in two
+// First / last uses of the tiles, the tile slots and the staging order.  The
+// slots fill 224 KB: fixed mode 14 of 16 KB, a slot per tile where a K-step has
+// no more tiles than that (7 + 7 digits), else rings (3 + 6 digits in two
 // K-blocks: the three-digit operand's six tiles live throughout, a window of
-// six of the other's); f32 mode 6 of 16 KB and 4 of 32 KB.
+// six of the other's); f32 mode rings of 6 of 16 KB and 4 of 32 KB.
+constexpr int kFixedSlots = 14;
 void plan_pairs(TcParams& p, int mode) {
   for (int i = 0; i < p.npairs; ++i) {
     TcPair& pr = p.pairs[i];
@@ -796,12 +821,25 @@ void plan_pairs(TcParams& p, int mode) {
                          (lastA ? kPairLastA : 0) | (lastB ? kPairLastB : 0));
   }
   if (p.kspan == 2) p.kblocks = (p.kblocks + 1) / 2;     // a step past K' reads zeros
-  if (mode == 0) {
+  const int ta = p.planes_a * p.kspan, tb = p.planes_b * p.kspan;
+  const bool resident = mode == 0 && ta + tb <= kFixedSlots && ta <= MAX_SLOTS && tb <= MAX_SLOTS;
+  if (resident) {
+    p.slots_a = ta;
+    p.slots_b = tb;
+  } else if (mode == 0) {
     p.slots_a = p.planes_a < p.planes_b ? 6 : p.planes_a > p.planes_b ? 8 : 7;
-    p.slots_b = 14 - p.slots_a;
+    p.slots_b = kFixedSlots - p.slots_a;
   } else {
     p.slots_a = 6;
     p.slots_b = 4;
+  }
+  // staging order: a slot per tile is free again after its tile's last use in
+  // the step before; slots in rings are filled in the order of first use
+  p.nload = 0;
+  const int want = resident ? kPairLastA : kPairFirstA, wantb = resident ? kPairLastB : kPairFirstB;
+  for (int i = 0; i < p.npairs; ++i) {
+    if (p.pairs[i].flags & want) p.load[p.nload++] = p.pairs[i].pa;
+    if (p.pairs[i].flags & wantb) p.load[p.nload++] = (int8_t)(-1 - p.pairs[i].pb);
   }
 }
 
@@ -834,12 +872,12 @@ int launch(olc_context* ctx, int mode, const void* dA, const void* dB, int plane
     if ((s = cuda_check(cudaFuncSetAttribute(tc_gemm_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem),
                         "tc smem")))
       return s;
-    tc_gemm_kernel<0><<<grid, num_threads<0>(), smem, st>>>(ta, tb, p);
+    tc_gemm_kernel<0><<<grid, kThreads, smem, st>>>(ta, tb, p);
   } else {
     if ((s = cuda_check(cudaFuncSetAttribute(tc_gemm_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem),
                         "tc smem")))
       return s;
-    tc_gemm_kernel<1><<<grid, num_threads<1>(), smem, st>>>(ta, tb, p);
+    tc_gemm_kernel<1><<<grid, kThreads, smem, st>>>(ta, tb, p);
   }
   count_launch();
   double frac = 1.0;
@@ -887,8 +925,6 @@ int zgemm_fixed(olc_context* ctx, int m, int n, int k, const TA* A, long long sA
   fixed_plan(bits_a, bits_b, std::max(bits_a, bits_b), &na, &nbd, &T);
   const int kp = (k + 31) & ~31;
   const size_t Kp = 2 * (size_t)kp;
-  // one group per weight s + t = d <= T, its pairs with A's new plane first and
-  // B's last (planes enter in the order 0, 1, ..)
   TcParams plan{};
   // 64-bit fixed point: unit 2^(L - beta (T + 2)) of the scale product
   const double mag = kBeta * T + 2 * kBeta + std::log2(1.03 * (double)Kp);
@@ -898,13 +934,26 @@ int zgemm_fixed(olc_context* ctx, int m, int n, int k, const TA* A, long long sA
   // (a drain of the 128 x 128 tile takes the epilogue 1600 clocks, three pairs of
   // one K-block the tensor cores 950).
   plan.kspan = std::min(na, nbd) <= 3 ? 2 : 1;
-  for (int d = 0; d <= T; ++d) {
-    const int first = plan.npairs;
-    for (int s = std::min(d, na - 1); s >= 0 && d - s < nbd; --s)
+  // One group per weight s + t = d <= T.  Where every tile of a K-step has a slot of
+  // its own, from the highest weight down and its pairs from the middle out: the
+  // low-order tiles retire first and the tiles that the next step begins with long
+  // before its first pair (from weight 0 up all tiles retired in the last group and
+  // every step began with a wait for its copies).  In
+  // rings the pairs run from weight 0 up, A's new plane first and B's last, so that
+  // tiles are used in the order 0, 1, ..
+  const bool down = (na + nbd) * plan.kspan <= kFixedSlots && std::max(na, nbd) * plan.kspan <= MAX_SLOTS;
+  for (int g = 0; g <= T; ++g) {
+    const int d = down ? T - g : g, first = plan.npairs;
+    int order[32], cnt = 0;
+    for (int q = std::min(d, na - 1); q >= 0 && d - q < nbd; --q) order[cnt++] = q;
+    if (down)
+      std::stable_sort(order, order + cnt, [d](int x, int y) { return std::abs(2 * x - d) < std::abs(2 * y - d); });
+    for (int j = 0; j < cnt; ++j)
       for (int q = 0; q < plan.kspan; ++q) {
         if (plan.npairs == kMaxPairs || plan.ngroups == kMaxGroups)
           return fail(OLC_ERR_UNSUPPORTED, "fixed-point product: too many digit pairs");
-        plan.pairs[plan.npairs++] = TcPair{(int8_t)(plan.kspan * s + q), (int8_t)(plan.kspan * (d - s) + q), 0};
+        plan.pairs[plan.npairs++] =
+            TcPair{(int8_t)(plan.kspan * order[j] + q), (int8_t)(plan.kspan * (d - order[j]) + q), 0};
       }
     if (plan.npairs == first) continue;
     plan.pairs[first].flags |= kPairStart;

@@ -11,10 +11,11 @@ namespace tc {
 constexpr int kBeta = 8;         // bits per digit of the fixed-point split (exact in BF16)
 constexpr int kMaxPairs = 96;    // digit pairs (or BF16-piece pairs) per launch
 constexpr int kMaxGroups = 24;   // groups of pairs that share an accumulator
+constexpr int kMaxTiles = 32;    // operand tiles of a K-step
 
 // One pair of operand tiles of a launch, in the order the pairs run within a
-// K-step of kspan K-blocks; pa, pb: tiles in the order of their first use in the
-// step (tile j = plane j / kspan of K-block j % kspan of the step).  flags: kPair*.
+// K-step of kspan K-blocks; pa, pb: tiles (tile j = plane j / kspan of K-block
+// j % kspan of the step).  flags: kPair*.
 struct TcPair {
   int8_t pa, pb;
   int16_t flags;
@@ -45,6 +46,8 @@ struct TcParams {
   int tri_a_upper, tri_a_lower, tri_b_upper;   // triangular operands: zero K blocks skipped
   int* err;                     // device error word (expired waits)
   TcPair pairs[kMaxPairs];
+  int nload;                    // tiles of a K-step
+  int8_t load[kMaxTiles];       // in the order they are staged: tile of A, or -1 - tile of B
   int16_t shift[kMaxGroups];    // fixed mode: int64 shift of a group's drained sums (negative: right)
 };
 
