@@ -38,7 +38,11 @@ int launch_class(olc_context* ctx, int cls, const double* coeffs, int ep_type, i
   a.ep_type = ep_type;
   a.ep_alpha = ep_alpha;
   if (a.n == 0) return OLC_OK;
-  const dim3 block(kThirdThreads), grid((a.n + kThirdThreads - 1) / kThirdThreads);
+  a.log_split = 0;
+  if (OP == OLC_OP_NUCLEAR || OP == OLC_OP_ELECPOT)
+    while (a.log_split < 5 && ((long long)a.n << (a.log_split + 1)) <= kThirdWave) ++a.log_split;
+  const dim3 block(kThirdThreads),
+      grid((unsigned)((((long long)a.n << a.log_split) + kThirdThreads - 1) / kThirdThreads));
   StageScope scope(ctx, OLC_STAGE_PRIMITIVES);
   const int l1 = cls / (kMaxL + 1), l2 = cls % (kMaxL + 1);
   if (l1 == 3 || l2 == 3) {

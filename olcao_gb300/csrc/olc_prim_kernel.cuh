@@ -61,6 +61,7 @@ struct PrimArgs {
   int accumulate;
   int ep_type;              // EP: potential type of a single term, -1 = all types
   int ep_alpha;             // EP: exponent index of a single term
+  int log_split;            // third-centre operators: log2 of the lanes that share an item
 };
 
 // Two-centre operators, one thread per item.
@@ -110,8 +111,18 @@ __global__ void __launch_bounds__(128) prim_kernel(SysView v, PrimArgs a) {
 // are summed in FP32, in a queue and accumulators of their own, in the same
 // pass (all 16 terms of the 64-atom cell's d-d class: 109 ms in two passes
 // of Cartesian blocks before).
+//
+// Small systems have too few items for the chip (a two-atom cell's f-f class
+// 40 to 60 blocks): 2^log_split threads then share an item, as many as keep all
+// items in one wave of kThirdWave threads (two blocks an SM, the residency of
+// the f classes).  For one operator they are warps of a block first, so that one
+// full warp still transforms 32 items; where all potential terms are summed the
+// images outweigh the transformation and lanes, which even out the items'
+// image counts within a warp, are better (d-d class of a two-atom cell 4.4 ->
+// 1.4 ms, by warps 1.9 ms).  SPLIT_MS
 constexpr int kThirdThreads = 128;
 constexpr int kQueue = 16;
+constexpr int kThirdWave = 152 * 2 * kThirdThreads;
 
 template <int OP, int L1, int L2, bool FAR32>
 __global__ void __launch_bounds__(kThirdThreads) third_centre_kernel(SysView v, PrimArgs a) {
@@ -121,7 +132,14 @@ __global__ void __launch_bounds__(kThirdThreads) third_centre_kernel(SysView v, 
   __shared__ double exptab[64];
   if (threadIdx.x < 64) exptab[threadIdx.x] = kExp2Neg[threadIdx.x];
   __syncthreads();
-  const int idx = blockIdx.x * kThirdThreads + threadIdx.x, tid = threadIdx.x;
+  // split threads share an item and take its images in turn: the warps of a
+  // block first (2^lw), then neighbouring lanes (2^ll); lanes alone where all
+  // potential terms are summed
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int lw = a.ep_type < 0 && OP != OLC_OP_NUCLEAR ? 0 : min(a.log_split, 2);
+  const int ll = a.log_split - lw, split = 1 << a.log_split;
+  const int sub = ((warp & ((1 << lw) - 1)) << ll) | (lane & ((1 << ll) - 1));
+  const int idx = (int)((blockIdx.x * (kThirdThreads / 32) + warp) >> lw) * (32 >> ll) + (lane >> ll);
   const bool live = idx < a.n;
   ItemGeom g;
   const int atom = load_item(v, a.task[live ? idx : 0], a.ab[live ? idx : 0], g);
@@ -193,7 +211,7 @@ __global__ void __launch_bounds__(kThirdThreads) third_centre_kernel(SysView v, 
       const float reach = (ap + (float)sqrt(tad)) * 1.00001f;
       const float near2 = (float)tad + 1e-5f * reach * reach;
       const float rhoh = (float)rho, rhol = (float)(rho - (double)rhoh);
-      int c = i0;
+      int c = i0 + sub;
       bool more = true;
       while (more) {
         int cnt = 0, cntf = 0;
@@ -209,7 +227,7 @@ __global__ void __launch_bounds__(kThirdThreads) third_centre_kernel(SysView v, 
             if (FAR32 && rhoh * d2 > (float)kFarRho) farq[cntf++][tid] = c;
             else queue[cnt++][tid] = c;
           }
-          ++c;
+          c += split;
         }
         __syncwarp();
         for (int s = 0; s < cnt; ++s) {
@@ -272,7 +290,35 @@ __global__ void __launch_bounds__(kThirdThreads) third_centre_kernel(SysView v, 
       }
     }
   }
-  if (!live) return;
+  if (FAR32)
+#pragma unroll
+    for (int q = 0; q < NM; ++q) E[q] += (double)Ef[q];
+  for (int o = (1 << ll) >> 1; o; o >>= 1) {
+    any |= __shfl_xor_sync(0xffffffffu, any ? 1 : 0, o) != 0;
+#pragma unroll
+    for (int q = 0; q < NM; ++q) E[q] += __shfl_xor_sync(0xffffffffu, E[q], o);
+  }
+  if (lw) {
+    __shared__ double sums[NM][32];
+    __shared__ bool anys[32];
+    for (int w = 1; w < kThirdThreads / 32; ++w) {
+      const int first = w & ~((1 << lw) - 1);           // the warp that keeps the item's sum
+      if (first == w) continue;
+      if (warp == w) {
+        anys[lane] = any;
+#pragma unroll
+        for (int q = 0; q < NM; ++q) sums[q][lane] = E[q];
+      }
+      __syncthreads();
+      if (warp == first) {
+        any |= anys[lane];
+#pragma unroll
+        for (int q = 0; q < NM; ++q) E[q] += sums[q][lane];
+      }
+      __syncthreads();
+    }
+  }
+  if (!live || sub) return;
   double* out = a.out + (size_t)idx * NS;
   if (!any) {
     if (!a.accumulate)
@@ -280,16 +326,17 @@ __global__ void __launch_bounds__(kThirdThreads) third_centre_kernel(SysView v, 
       for (int q = 0; q < NS; ++q) out[q] = 0.0;
     return;
   }
-  if (FAR32)
-#pragma unroll
-    for (int q = 0; q < NM; ++q) E[q] += (double)Ef[q];
   if (single) {
     const double a3 = v.pot_types[a.ep_type].alphas[a.ep_alpha], iz3 = 1.0 / (z + a3);
     monomials_to_moments<LT>(a3 * iz3, 0.5 * iz3, E);
   }
-  double cart[N1 * N2];
-  moments_to_cart<L1, L2>(E, PA, PB, cart);
-  store_harmonic<L1, L2, double>(cart, out, a.accumulate != 0, 1.0);
+  if constexpr (LT >= 6) {
+    moments_to_harmonics<L1, L2>(E, PA, PB, out, a.accumulate != 0);
+  } else {
+    double cart[N1 * N2];
+    moments_to_cart<L1, L2>(E, PA, PB, cart);
+    store_harmonic<L1, L2, double>(cart, out, a.accumulate != 0, 1.0);
+  }
 }
 
 // One primitive of explicit inputs (the testing entry olc_primitive_batch).

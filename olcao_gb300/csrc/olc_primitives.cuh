@@ -13,6 +13,7 @@
 // (gaussIntegrals.f90:16080-16221, see boys_reference below).
 #pragma once
 
+#include <utility>
 #include <cuda_runtime.h>
 
 namespace olc {
@@ -535,6 +536,135 @@ __device__ __forceinline__ void moments_to_cart(const double* E, const double (&
             }
         }
     }
+}
+
+// Harmonic P of a Cartesian line: get(i) is component i.
+template <int P, class G>
+__device__ __forceinline__ double harmonic(G get) {
+  static_assert(hn(P) <= 3, "harmonics have up to three terms");
+  double v = hw(P, 0) == 1.0 ? get(hc(P, 0)) : hw(P, 0) * get(hc(P, 0));
+  if constexpr (hn(P) > 1) v = fma(hw(P, 1), get(hc(P, 1)), v);
+  if constexpr (hn(P) > 2) v = fma(hw(P, 2), get(hc(P, 2)), v);
+  return v;
+}
+template <class G, class Put, int... P>
+__device__ __forceinline__ void harmonics(G get, Put put, std::integer_sequence<int, P...>) {
+  (put(P, harmonic<P>(get)), ...);
+}
+// cidx by table, for loops that are not unrolled
+constexpr signed char cidx_or_0(int x, int y, int z) { return (signed char)(x + y + z <= 3 ? cidx(x, y, z) : 0); }
+static __device__ const signed char kCidx[4][4][4] = {
+#define OLC_CROW(x, y) {cidx_or_0(x, y, 0), cidx_or_0(x, y, 1), cidx_or_0(x, y, 2), cidx_or_0(x, y, 3)}
+#define OLC_CPLANE(x) {OLC_CROW(x, 0), OLC_CROW(x, 1), OLC_CROW(x, 2), OLC_CROW(x, 3)}
+    OLC_CPLANE(0), OLC_CPLANE(1), OLC_CPLANE(2), OLC_CPLANE(3)};
+#undef OLC_CPLANE
+#undef OLC_CROW
+
+// moments_to_cart and store_harmonic of the f-f class: some 2600 FP64
+// instructions an item as loops over arrays in local memory.  That class outgrows
+// the compiler's unrolling (7 KB of arrays indexed by evaluated formulas): 0.51 ms
+// for the items of a two-atom cell, nearly all of it here, against 0.35 ms with
+// these loops.  d-f still unrolls: 0.10 ms an f-d launch, as loops 0.18 ms.
+template <int L1, int L2>
+__device__ __forceinline__ void moments_to_harmonics(const double* E, const double (&PA)[3], const double (&PB)[3],
+                                                     double* out, bool accumulate) {
+  constexpr int LT = L1 + L2, N1 = ncart(L1), N2 = ncart(L2), NS1 = nharm(L1), NS2 = nharm(L2), W = LT + 1;
+  double M[nmom(LT)];                     // the moments, indexed by loops
+#pragma unroll
+  for (int q = 0; q < nmom(LT); ++q) M[q] = E[q];
+  double c[3][L1 + 1][L2 + 1][W];         // (y + PA)^a (y + PB)^b = sum_i c[a][b][i] y^i
+#pragma unroll 1
+  for (int d = 0; d < 3; ++d) {
+    const double pa = PA[d], pb = PB[d];
+#pragma unroll 1
+    for (int a = 0; a <= L1; ++a)
+#pragma unroll 1
+      for (int b = 0; b <= L2; ++b) {
+        double* o = c[d][a][b];
+        if (a + b == 0) {
+          o[0] = 1.0;
+          continue;
+        }
+        const double* low = a > 0 ? c[d][a - 1][b] : c[d][a][b - 1];
+        const double w = a > 0 ? pa : pb;
+        double prev = 0.0;
+#pragma unroll 1
+        for (int i = 0; i < a + b; ++i) {
+          const double x = low[i];
+          o[i] = fma(w, x, prev);
+          prev = x;
+        }
+        o[a + b] = prev;
+      }
+  }
+  double cart[N1 * N2];
+#pragma unroll 1
+  for (int az = 0; az <= L1; ++az)
+#pragma unroll 1
+    for (int bz = 0; bz <= L2; ++bz) {
+      const int r = az + bz, rz = LT - r;
+      const double* cz = c[2][az][bz];
+      double F[W * W];
+      int o = 0;
+#pragma unroll 1
+      for (int x = 0; x <= LT; ++x)
+#pragma unroll 1
+        for (int y = 0; y <= LT - x; ++y) {
+          if (x + y <= rz) {
+            double v = M[o + r];
+#pragma unroll 2
+            for (int k = 0; k < r; ++k) v = fma(cz[k], M[o + k], v);
+            F[x * W + y] = v;
+          }
+          o += W - x - y;
+        }
+#pragma unroll 1
+      for (int ay = 0; ay <= L1 - az; ++ay)
+#pragma unroll 1
+        for (int by = 0; by <= L2 - bz; ++by) {
+          const int s = ay + by, ry = rz - s;
+          const double* cy = c[1][ay][by];
+          double G[W];
+#pragma unroll 1
+          for (int x = 0; x <= ry; ++x) {
+            double v = F[x * W + s];
+#pragma unroll 2
+            for (int k = 0; k < s; ++k) v = fma(cy[k], F[x * W + k], v);
+            G[x] = v;
+          }
+#pragma unroll 1
+          for (int ax = 0; ax <= L1 - az - ay; ++ax)
+#pragma unroll 1
+            for (int bx = 0; bx <= L2 - bz - by; ++bx) {
+              const double* cx = c[0][ax][bx];
+              double v = G[ax + bx];
+#pragma unroll 2
+              for (int k = 0; k < ax + bx; ++k) v = fma(cx[k], G[k], v);
+              cart[kCidx[ax][ay][az] * N2 + kCidx[bx][by][bz]] = v;
+            }
+        }
+    }
+  // harmonics of the first index in place (NS1 <= N1 rows), then of the second
+#pragma unroll 1
+  for (int b = 0; b < N2; ++b) {
+    double line[N1];
+#pragma unroll
+    for (int a = 0; a < N1; ++a) line[a] = cart[a * N2 + b];
+    harmonics([&](int a) { return line[a]; }, [&](int p, double v) { cart[p * N2 + b] = v; },
+              std::make_integer_sequence<int, NS1>());
+  }
+#pragma unroll 1
+  for (int p = 0; p < NS1; ++p) {
+    double line[N2];
+#pragma unroll
+    for (int b = 0; b < N2; ++b) line[b] = cart[p * N2 + b];
+    harmonics([&](int b) { return line[b]; },
+              [&](int q, double v) {
+                double* o = out + q * NS1 + p;
+                *o = accumulate ? *o + v : v;
+              },
+              std::make_integer_sequence<int, NS2>());
+  }
 }
 
 // Far-shell split of the electronic potential.  With rho = z a3 / z3 |P - C|^2
