@@ -455,7 +455,8 @@ __global__ void assemble_full_kernel(const double* __restrict__ terms, const dou
        idx += (size_t)gridDim.x * blockDim.x) {
     const int k = (int)(idx / plen);
     const size_t r = idx % plen;
-    int i = (int)((sqrt(8.0 * (double)r + 1.0) - 1.0) * 0.5);
+    // an estimate in FP32, corrected: FP64 instructions bound this kernel
+    int i = (int)((sqrtf(8.f * (float)(long long)r + 1.f) - 1.f) * 0.5f);
     while ((size_t)i * (i + 1) / 2 > r) --i;
     while ((size_t)(i + 1) * (i + 2) / 2 <= r) ++i;
     const int j = (int)(r - (size_t)i * (i + 1) / 2);
