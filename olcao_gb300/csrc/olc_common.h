@@ -161,6 +161,7 @@ struct olc_context {
   double* d_work_cv = nullptr;
   double* d_work_cc = nullptr;
   double* d_work_x = nullptr;      // GEMM temporaries
+  double* d_work_p = nullptr;
   double* d_work_w = nullptr;
   void* d_solver_work = nullptr;
   size_t solver_work_bytes = 0;

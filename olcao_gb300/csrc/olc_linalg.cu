@@ -101,10 +101,29 @@ __global__ void __launch_bounds__(256) ortho_pack_kernel(PackArgs a) {
   }
 }
 
-// W = O_cv - W / 2 with W = O_cc S_cv on entry
-__global__ void core_fold_kernel(const double* __restrict__ cv, double* __restrict__ w, size_t len) {
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < len; i += (size_t)gridDim.x * blockDim.x)
-    w[i] = cv[i] - 0.5 * w[i];
+// W = O_cv - (S_cv^H O_cc)^H / 2 (nc x nv) from the product P = S_cv^H O_cc
+// (nv x nc): 32 x 32 tiles of P turned in shared memory.
+__global__ void __launch_bounds__(256) core_fold_kernel(const double2* __restrict__ cv, const double2* __restrict__ P,
+                                                        int nc, int nv, int nk, double2* __restrict__ W) {
+  __shared__ double2 tile[kPackTile][kPackTile + 1];
+  const int tc = (nc + kPackTile - 1) / kPackTile, tv = (nv + kPackTile - 1) / kPackTile;
+  const int lane = threadIdx.x & 31, row0 = threadIdx.x >> 5;
+  const long long total = (long long)tc * tv * nk;
+  for (long long b = blockIdx.x; b < total; b += gridDim.x) {
+    const size_t base = (size_t)(b / ((long long)tc * tv)) * nc * nv;
+    const int r = (int)(b % ((long long)tc * tv)), c0 = (r % tc) * kPackTile, v0 = (r / tc) * kPackTile;
+    __syncthreads();                         // the last tile is read
+    for (int q = row0; q < kPackTile; q += 8)
+      if (c0 + q < nc && v0 + lane < nv) tile[q][lane] = P[base + (size_t)(c0 + q) * nv + v0 + lane];
+    __syncthreads();
+    for (int q = row0; q < kPackTile; q += 8)
+      if (v0 + q < nv && c0 + lane < nc) {
+        const size_t at = base + (size_t)(v0 + q) * nc + c0 + lane;
+        const double* o = reinterpret_cast<const double*>(cv) + 2 * at;   // the caller's: any 8-byte address
+        const double2 p = tile[lane][q];
+        W[at] = make_double2(o[0] - 0.5 * p.x, o[1] + 0.5 * p.y);
+      }
+  }
 }
 
 // packed [nk][plen][2] -> full Hermitian [nk][n][n] (both triangles)
@@ -197,6 +216,7 @@ int ortho_pack_ex(olc_context* ctx, bool is_overlap, const double* vv, const dou
     const size_t nn = (size_t)nv * nv, ncv = 2 * (size_t)nv * nc * nk;
     if (!ctx->d_work_x) {
       if ((st = dalloc(ctx, &ctx->d_work_x, 2 * nn * nk))) return st;
+      if ((st = dalloc(ctx, &ctx->d_work_p, ncv))) return st;
       if ((st = dalloc(ctx, &ctx->d_work_w, ncv))) return st;
     }
     // both products on the tensor cores, FP64-accurate (split digits,
@@ -204,11 +224,18 @@ int ortho_pack_ex(olc_context* ctx, bool is_overlap, const double* vv, const dou
     int bits = 53;
     if (const char* v = std::getenv("OLC_ORTHO_BITS")) bits = std::max(24, std::min(53, std::atoi(v)));
     const long long sCV = 2LL * nc * nv, sCC = 2LL * nc * nc;
-    if ((st = ozaki_zgemm<double, double>(ctx, nc, nv, nc, cc, sCC, nc, false, bits, scv, sCV, nc, bits,
-                                          ctx->d_work_w, nk, OLC_STAGE_ORTHO))) return st;
+    // (O_cc S_cv)^H: with the long side in rows of 128 the tiles pad less than
+    // O_cc S_cv's (n_c = 320, n_v = 832 at 8 k-points: 280 tiles, two waves, not
+    // 312, a third wave for eight of them; both products of 19 operators 18.9 ->
+    // 16.9 ms)
+    if ((st = ozaki_zgemm<double, double>(ctx, nv, nc, nc, scv, sCV, nc, true, bits, cc, sCC, nc, bits,
+                                          ctx->d_work_p, nk, OLC_STAGE_ORTHO))) return st;
     {
       StageScope scope(ctx, OLC_STAGE_ORTHO);
-      core_fold_kernel<<<grid_for(ncv), 256, 0, ctx->stream>>>(is_overlap ? scv : cv, ctx->d_work_w, ncv);
+      const size_t tiles = (size_t)((nc + kPackTile - 1) / kPackTile) * ((nv + kPackTile - 1) / kPackTile) * nk;
+      core_fold_kernel<<<(int)std::min<size_t>(tiles, 152 * 32), 256, 0, ctx->stream>>>(
+          reinterpret_cast<const double2*>(is_overlap ? scv : cv), reinterpret_cast<const double2*>(ctx->d_work_p), nc,
+          nv, nk, reinterpret_cast<double2*>(ctx->d_work_w));
     }
     if ((st = ozaki_zgemm<double, double>(ctx, nv, nv, nc, scv, sCV, nc, true, bits, ctx->d_work_w, sCV, nc,
                                           bits, ctx->d_work_x, nk, OLC_STAGE_ORTHO))) return st;
