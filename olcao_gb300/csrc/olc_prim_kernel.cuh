@@ -119,7 +119,8 @@ __global__ void __launch_bounds__(128) prim_kernel(SysView v, PrimArgs a) {
 // full warp still transforms 32 items; where all potential terms are summed the
 // images outweigh the transformation and lanes, which even out the items'
 // image counts within a warp, are better (d-d class of a two-atom cell 4.4 ->
-// 1.4 ms, by warps 1.9 ms).  SPLIT_MS
+// 1.4 ms, by warps 1.9 ms).  With the f-f transformation as loops, the
+// third-centre kernels of a two-atom oxide's set-up took 26 ms, 33 before.
 constexpr int kThirdThreads = 128;
 constexpr int kQueue = 16;
 constexpr int kThirdWave = 152 * 2 * kThirdThreads;
