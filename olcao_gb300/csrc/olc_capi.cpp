@@ -158,6 +158,12 @@ int olc_destroy(olc_context_t* ctx) {
     cudaStreamDestroy(ctx->mixed_streams[i]);
     cudaEventDestroy(ctx->mixed_join[i]);
   }
+  for (cudaStream_t st : ctx->prim_streams) {
+    cudaStreamSynchronize(st);
+    cudaStreamDestroy(st);
+  }
+  for (cudaEvent_t e : ctx->prim_join) cudaEventDestroy(e);
+  if (ctx->prim_fork) cudaEventDestroy(ctx->prim_fork);
   if (ctx->ev_fork) cudaEventDestroy(ctx->ev_fork);
   if (ctx->graph_exec) cudaGraphExecDestroy(ctx->graph_exec);
   if (ctx->pool) {

@@ -172,6 +172,9 @@ struct olc_context {
   std::vector<double*> sub_eval;
   size_t sub_work_bytes = 0;
   int sub_n = 0;
+  std::vector<cudaStream_t> prim_streams;   // side streams of the third-centre classes
+  std::vector<cudaEvent_t> prim_join;
+  cudaEvent_t prim_fork = nullptr;
   cudaEvent_t ev_fork = nullptr;
   std::vector<cudaEvent_t> ev_join;
   // FP32 solves of the mixed-precision path
