@@ -555,12 +555,17 @@ static __device__ __noinline__ void hegv_reduced(cd* U, cd* C, cd* W, cd* T, int
   refine(C, U, W, T, n, ld, sh, trace);
 }
 
-// Ascending order of sh.w into sh.order (ties by index).
+// Ascending order of sh.w into sh.order, ties by index and NaN (of a matrix that
+// holds one) after every number: order is a permutation whatever w holds.
 static __device__ __forceinline__ void sorted_order(int n, Shared& sh) {
   for (int i = threadIdx.x; i < n; i += blockDim.x) {
     const double wi = sh.w[i];
     int rank = 0;
-    for (int j = 0; j < n; ++j) rank += sh.w[j] < wi || (sh.w[j] == wi && j < i);
+    for (int j = 0; j < n; ++j) {
+      const double wj = sh.w[j];
+      const bool tie = wj == wi || (isnan(wj) && isnan(wi));
+      rank += wj < wi || (isnan(wi) && !isnan(wj)) || (tie && j < i);
+    }
     sh.order[rank] = i;
   }
   __syncthreads();
