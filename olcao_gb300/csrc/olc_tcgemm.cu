@@ -437,9 +437,10 @@ __global__ void __launch_bounds__(kThreads, 1)
           } else {
             // low-order digit groups: rounded to the accumulator's unit (a
             // plain arithmetic shift would floor, a bias of half a unit per
-            // drain that adds up over long K)
-            const int half = 1 << (-sh - 1);
-            drain([sh, half](long long& x, int v) { x += (v + half) >> (-sh); });
+            // drain that adds up over long K).  |v| < 2^24, so that a shift by 26
+            // and more gives 0, and one past 30 (K of a million) may stop there
+            const int right = min(-sh, 30), half = 1 << (right - 1);
+            drain([right, half](long long& x, int v) { x += (v + half) >> right; });
           }
         }
       }
