@@ -294,6 +294,12 @@ __global__ void __launch_bounds__(kThirdThreads) third_centre_kernel(SysView v, 
   if (FAR32)
 #pragma unroll
     for (int q = 0; q < NM; ++q) E[q] += (double)Ef[q];
+  // two exponents past their element's table have no screen: no number, not 0
+  if (ap != ap) {
+    any = true;
+#pragma unroll
+    for (int q = 0; q < NM; ++q) E[q] = (double)ap;
+  }
   for (int o = (1 << ll) >> 1; o; o >>= 1) {
     any |= __shfl_xor_sync(0xffffffffu, any ? 1 : 0, o) != 0;
 #pragma unroll

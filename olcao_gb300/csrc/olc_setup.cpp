@@ -135,6 +135,11 @@ void make_images(const Lattice& lat, const olc_context* ctx, const std::vector<i
                  const std::vector<double>& sitePos, const double* potPos, const std::vector<double>& elemAlpha,
                  const std::vector<double>& elemPot, const std::vector<double>& elemNuc, double T, Images& im) {
   const int ns = (int)siteType.size();
+  // an atom type with more exponents than its element's first type: the table holds
+  // 0 for them, the screen's centre lies on B' and its radius is B's own
+  double minAlpha = HUGE_VAL, maxSep = 0.0;
+  for (const DevType& t : ctx->htypes) minAlpha = std::min(minAlpha, elemAlpha[(size_t)t.element * OLC_MAX_ALPHAS]);
+  for (const DevTask& t : ctx->htasks) maxSep = std::max(maxSep, t.sep);
   double plane[3];            // spacing of the lattice planes, inverted
   for (int l = 0; l < 3; ++l)
     plane[l] = std::sqrt(lat.inv[l][0] * lat.inv[l][0] + lat.inv[l][1] * lat.inv[l][1] + lat.inv[l][2] * lat.inv[l][2]);
@@ -150,7 +155,10 @@ void make_images(const Lattice& lat, const olc_context* ctx, const std::vector<i
       if (pt.nuc_charge >= 1.0e-8) a3 = std::min(a3, elemNuc[pt.element]);
       // an exponent of 0 (a bare charge, a type with more terms than its
       // element's table) has no radius: every image of the cell list's extent
-      double rad = std::sqrt(T * (1.0 / a1 + 1.0 / a3)) * (1.0 + 1e-6);
+      double rad = std::sqrt(T * (1.0 / a1 + 1.0 / a3));
+      if (elemAlpha[(size_t)t1.element * OLC_MAX_ALPHAS + t1.nalpha - 1] == 0.0)
+        rad = std::sqrt(maxSep) + std::sqrt(T * (1.0 / minAlpha + 1.0 / a3));
+      rad *= 1.0 + 1e-6;
       if (!(a3 > 0.0) || !(rad < 1e6)) rad = std::sqrt(lat.cells.back());
       const double rad2 = rad * rad;
       found.clear();
@@ -431,10 +439,18 @@ int build_system(olc_context* ctx, const olc_system_t* s) {
     for (int y = 0; y < s->num_atom_types; ++y) {
       const DevType &t1 = ctx->htypes[x], &t2 = ctx->htypes[y];
       auto& tp = typePairs[(size_t)x * s->num_atom_types + y];
-      for (int a1 = 0; a1 < t1.nalpha; ++a1)
-        for (int a2 = 0; a2 < t2.nalpha; ++a2)
-          tp.push_back({alphaDist(a1, a2, t1.element, t2.element), t1.alphas[a1] + t2.alphas[a2],
-                        t1.lmax_alpha[a1] * (kMaxL + 1) + t2.lmax_alpha[a2], a1 | (a2 << 8)});
+      for (int a1 = 0; a1 < t1.nalpha; ++a1) {
+        // the row of a1 ends at its first pair out of reach: every pair is held to the
+        // smallest radius up to it (past the exponents of an element's first type
+        // the radius is not defined and the table gives infinity)
+        double dist = HUGE_VAL;
+        for (int a2 = 0; a2 < t2.nalpha; ++a2) {
+          const double d = alphaDist(a1, a2, t1.element, t2.element);
+          if (d < dist) dist = d;
+          tp.push_back({dist, t1.alphas[a1] + t2.alphas[a2], t1.lmax_alpha[a1] * (kMaxL + 1) + t2.lmax_alpha[a2],
+                        a1 | (a2 << 8)});
+        }
+      }
       std::stable_sort(tp.begin(), tp.end(), [](const AlphaPair& p, const AlphaPair& q) { return p.sum < q.sum; });
     }
   std::vector<int32_t> itTask[kNumClasses], itAB[kNumClasses], itStart[kNumClasses];
