@@ -87,6 +87,12 @@ __global__ void __launch_bounds__(128) prim_kernel(SysView v, PrimArgs a) {
   store_harmonic<L1, L2, double>(cart, a.out + (size_t)idx * NS, a.accumulate != 0, 1.0);
 }
 
+// |S - C'|^2 <= radius^2 for the image D = C' - A and S = PS + A.
+__device__ __forceinline__ bool within(const double4_16a& D, const double (&PS)[3], double tad) {
+  const double y[3] = {PS[0] - D.x, PS[1] - D.y, PS[2] - D.z};
+  return y[0] * y[0] + y[1] * y[1] + y[2] * y[2] <= tad;
+}
+
 // Third-centre operators (nuclear attraction, electronic potential), one
 // thread per item: the moments about P summed over the images within the
 // reference's radius (the image set of integrals.F90:2374-2418, 2533-2594),
@@ -107,8 +113,8 @@ __global__ void __launch_bounds__(128) prim_kernel(SysView v, PrimArgs a) {
 // place of the moments' recurrences (75 FP64 instructions a d-d image, not 94):
 // 1.65 ms a d-d term of the 64-atom cell, f-f and nuclear as before.
 //
-// FAR32 (mixed precision): images whose suppression is below exp(-kFarRho)
-// are summed in FP32, in a queue and accumulators of their own, in the same
+// FAR32 (mixed precision): images whose suppression exp(-rho |P - C'|^2) about the
+// pair's own centre is below exp(-kFarRho) are summed in FP32, in a queue and accumulators of their own, in the same
 // pass (all 16 terms of the 64-atom cell's d-d class: 109 ms in two passes
 // of Cartesian blocks before).
 //
@@ -211,6 +217,8 @@ __global__ void __launch_bounds__(kThirdThreads) third_centre_kernel(SysView v, 
       // up to it are good to 1e-6 of it)
       const float reach = (ap + (float)sqrt(tad)) * 1.00001f;
       const float near2 = (float)tad + 1e-5f * reach * reach;
+      // far images take the exact test here, where the margin leaves it open
+      const float sure2 = (float)tad - 1e-5f * reach * reach;
       const float rhoh = (float)rho, rhol = (float)(rho - (double)rhoh);
       int c = i0 + sub;
       bool more = true;
@@ -225,8 +233,20 @@ __global__ void __launch_bounds__(kThirdThreads) third_centre_kernel(SysView v, 
           const float x = psf[0] - q.x, y = psf[1] - q.y, w = psf[2] - q.z;
           const float d2 = x * x + y * y + w * w;
           if (d2 <= near2) {
-            if (FAR32 && rhoh * d2 > (float)kFarRho) farq[cntf++][tid] = c;
-            else queue[cnt++][tid] = c;
+            bool far = false;
+            if (FAR32) {
+              float p2 = d2;                               // |P - C'|^2, the suppression's
+              if (!same) {
+                const float px = pah[0] - q.x, py = pah[1] - q.y, pz = pah[2] - q.z;
+                p2 = px * px + py * py + pz * pz;
+              }
+              far = rhoh * p2 > (float)kFarRho;
+            }
+            if (!far) {
+              queue[cnt++][tid] = c;
+            } else if (d2 <= sure2 || within(v.img_d[c], PS, tad)) {
+              farq[FAR32 ? cntf++ : 0][FAR32 ? tid : 0] = c;
+            }
           }
           c += split;
         }
