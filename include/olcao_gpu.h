@@ -169,8 +169,9 @@ int olc_gauss_overlap(olc_context_t* ctx, int op, int term,
 
 /* Orthogonalise and pack, for all k (DEVICE arrays).  For the overlap
  * operator pass cv == s_cv.  Outputs packed[2, packed_len, nk] with the
- * reference's |x| < 1e-10 flush when core_dim > 0. vv is overwritten.  cc is
- * Hermitian, as an operator's core block is (only its Hermitian part enters). */
+ * reference's |x| < 1e-10 flush when core_dim > 0. vv is overwritten.  A
+ * cc that is not Hermitian to 2^-44 of its largest component enters as it is,
+ * by a slower product. */
 int olc_ortho_pack(olc_context_t* ctx, int is_overlap, double* vv,
                    const double* cv, const double* cc, const double* s_cv,
                    double* packed);

@@ -82,9 +82,8 @@ int cuda_check(cudaError_t e, const char* what) {
 int build_phase_table(olc_context* ctx);
 int ozaki_selftest(olc_context* ctx, int m, int n, int k, const double* A, const double* B,
                    double* C);
-int ortho_pack_ex(olc_context* ctx, bool is_overlap, const double* vv, const double* cv,
-                  const double* cc, const double* scv, double* packed, double* full,
-                  const double* add);
+int ortho_pack_blocks(olc_context* ctx, bool is_overlap, const double* vv, const double* cv, const double* cc,
+                      const double* scv, double* packed);
 
 }  // namespace olc
 
@@ -222,10 +221,7 @@ int olc_ortho_pack(olc_context_t* ctx, int is_overlap, double* vv, const double*
   if (!ctx || !vv || !packed) return fail(OLC_ERR_ARG, "olc_ortho_pack: null argument");
   if (ctx->dims.core_dim && (!cv || !cc || !s_cv))
     return fail(OLC_ERR_ARG, "olc_ortho_pack: core blocks required");
-  int st = ortho_pack_ex(ctx, is_overlap != 0, vv, cv, cc, is_overlap ? cv : s_cv, packed,
-                         nullptr, nullptr);
-  if (st) return st;
-  return cuda_check(cudaStreamSynchronize(ctx->stream), "olc_ortho_pack sync");
+  return ortho_pack_blocks(ctx, is_overlap != 0, vv, cv, cc, is_overlap ? cv : s_cv, packed);
 }
 
 int olc_assemble_hamiltonian(olc_context_t* ctx, const double* const* terms, const double* coeffs,

@@ -31,7 +31,8 @@ namespace {
 // combine, flush and pack; optionally also emit the full upper matrix (+ add)
 struct PackArgs {
   const double* vv;      // [nk][nv][nv]
-  const double* X;       // S_cv^H (O_cv - O_cc S_cv / 2)   (unused when nc == 0)
+  const double* X;       // S_cv^H (O_cv - O_cc S_cv / 2), S_cv^H O_cv with Y   (unused when nc == 0)
+  const double* Y;       // nullptr, or S_cv^H O_cc S_cv of an O_cc that is not Hermitian
   const double* add;     // optional full upper matrix added after the flush
   double* packed;        // [nk][plen][2] or nullptr
   double* full;          // [nk][nv][nv] upper, or nullptr
@@ -55,6 +56,7 @@ __global__ void __launch_bounds__(256) ortho_pack_kernel(PackArgs a) {
   const size_t plen = (size_t)a.nv * (a.nv + 1) / 2, nn = (size_t)a.nv * a.nv;
   const int lane = threadIdx.x & 31, row0 = threadIdx.x >> 5;
   const double2* X = reinterpret_cast<const double2*>(a.X);
+  const double2* Y = reinterpret_cast<const double2*>(a.Y);
   const double2* add = reinterpret_cast<const double2*>(a.add);
   double2* full = reinterpret_cast<double2*>(a.full);
   for (long long b = blockIdx.x; b < total; b += gridDim.x) {
@@ -81,6 +83,10 @@ __global__ void __launch_bounds__(256) ortho_pack_kernel(PackArgs a) {
         v.x -= x.x + m.x;
         v.y -= x.y - m.y;
         if (i == j) v.y = 0.0;
+        if (Y) {
+          v.x += Y[off].x;
+          v.y += Y[off].y;
+        }
         if (fabs(v.x) < 1.0e-10) v.x = 0.0;
         if (fabs(v.y) < 1.0e-10) v.y = 0.0;
       }
@@ -123,6 +129,41 @@ __global__ void __launch_bounds__(256) core_fold_kernel(const double2* __restric
         const double2 p = tile[lane][q];
         W[at] = make_double2(o[0] - 0.5 * p.x, o[1] + 0.5 * p.y);
       }
+  }
+}
+
+// Largest magnitudes of a component of O_cc and of O_cc - O_cc^H per k (as the bits
+// of doubles, which order like the non-negative numbers and NaN above them):
+// out[2 k], out[2 k + 1], zero on entry.  32 x 32 tiles of the lower triangle.
+__global__ void __launch_bounds__(256) core_asymmetry_kernel(const double* __restrict__ cc, int nc,
+                                                             unsigned long long* __restrict__ out) {
+  __shared__ double2 mirror[kPackTile][kPackTile + 1];
+  const int r0 = blockIdx.x * kPackTile, c0 = blockIdx.y * kPackTile;
+  if (c0 > r0) return;
+  const double* a = cc + 2 * (size_t)blockIdx.z * nc * nc;       // the caller's: any 8-byte address
+  const int lane = threadIdx.x & 31, row0 = threadIdx.x >> 5;
+  for (int q = row0; q < kPackTile; q += 8)
+    if (r0 + q < nc && c0 + lane < nc) {
+      const size_t at = 2 * ((size_t)(r0 + q) * nc + c0 + lane);                // (row c0 + lane, column r0 + q)
+      mirror[q][lane] = make_double2(a[at], a[at + 1]);
+    }
+  __syncthreads();
+  unsigned long long big = 0, off = 0;
+  const auto bits = [](double x) { return (unsigned long long)__double_as_longlong(fabs(x)); };
+  for (int q = row0; q < kPackTile; q += 8)
+    if (c0 + q < nc && r0 + lane < nc) {
+      const size_t at = 2 * ((size_t)(c0 + q) * nc + r0 + lane);
+      const double2 x = make_double2(a[at], a[at + 1]), m = mirror[lane][q];
+      big = max(max(big, max(bits(x.x), bits(x.y))), max(bits(m.x), bits(m.y)));
+      off = max(off, max(bits(x.x - m.x), bits(x.y + m.y)));
+    }
+  for (int o = 16; o; o >>= 1) {
+    big = max(big, __shfl_xor_sync(0xffffffffu, big, o));
+    off = max(off, __shfl_xor_sync(0xffffffffu, off, o));
+  }
+  if (lane == 0) {
+    atomicMax(&out[2 * blockIdx.z], big);
+    atomicMax(&out[2 * blockIdx.z + 1], off);
   }
 }
 
@@ -199,19 +240,21 @@ int grid_for(size_t n) {
 
 }  // namespace
 
-// Orthogonalise one operator for all k.  vv/cv/cc are the operator's blocks
-// (cc Hermitian, as an operator's core block is), scv is S_cv.  Writes packed
-// and/or full (upper, with `add` added).
+// Orthogonalise one operator for all k.  vv/cv/cc are the operator's blocks,
+// scv is S_cv.  Writes packed and/or full (upper, with `add` added).  cc is
+// Hermitian, as an operator's core block is, unless general_cc:
 //   S_cv^H O_cv + O_cv^H S_cv - S_cv^H O_cc S_cv = X + X^H,
 //   X = S_cv^H (O_cv - O_cc S_cv / 2),
 // and for the overlap, O_cv = S_cv, the same: one product of order nv besides
 // O_cc S_cv where the separate terms take two (with the pack kernel below,
-// 19 operators of order 832 at 8 k-points: set-up 104 -> 90 ms).
+// 19 operators of order 832 at 8 k-points: set-up 104 -> 90 ms).  general_cc: the
+// terms apart, the last as it is.
 int ortho_pack_ex(olc_context* ctx, bool is_overlap, const double* vv, const double* cv,
                   const double* cc, const double* scv, double* packed, double* full,
-                  const double* add) {
+                  const double* add, bool general_cc) {
   const int nv = ctx->dims.vale_dim, nc = ctx->dims.core_dim, nk = ctx->dims.num_kpoints;
   int st;
+  double* Y = nullptr;
   if (nc) {
     const size_t nn = (size_t)nv * nv, ncv = 2 * (size_t)nv * nc * nk;
     if (!ctx->d_work_x) {
@@ -230,19 +273,26 @@ int ortho_pack_ex(olc_context* ctx, bool is_overlap, const double* vv, const dou
     // 16.9 ms)
     if ((st = ozaki_zgemm<double, double>(ctx, nv, nc, nc, scv, sCV, nc, true, bits, cc, sCC, nc, bits,
                                           ctx->d_work_p, nk, OLC_STAGE_ORTHO))) return st;
-    {
+    const double* ocv = is_overlap ? scv : cv;
+    if (general_cc) {
+      if ((st = cuda_check(ctx_malloc(ctx, (void**)&Y, 16 * nn * nk, ctx->stream), "malloc S^H O_cc S"))) return st;
+      if ((st = ozaki_zgemm<double, double>(ctx, nv, nv, nc, ctx->d_work_p, sCV, nv, false, bits, scv, sCV, nc, bits, Y,
+                                            nk, OLC_STAGE_ORTHO))) return st;
+    } else {
       StageScope scope(ctx, OLC_STAGE_ORTHO);
       const size_t tiles = (size_t)((nc + kPackTile - 1) / kPackTile) * ((nv + kPackTile - 1) / kPackTile) * nk;
       core_fold_kernel<<<(int)std::min<size_t>(tiles, 152 * 32), 256, 0, ctx->stream>>>(
-          reinterpret_cast<const double2*>(is_overlap ? scv : cv), reinterpret_cast<const double2*>(ctx->d_work_p), nc,
-          nv, nk, reinterpret_cast<double2*>(ctx->d_work_w));
+          reinterpret_cast<const double2*>(ocv), reinterpret_cast<const double2*>(ctx->d_work_p), nc, nv, nk,
+          reinterpret_cast<double2*>(ctx->d_work_w));
+      ocv = ctx->d_work_w;
     }
-    if ((st = ozaki_zgemm<double, double>(ctx, nv, nv, nc, scv, sCV, nc, true, bits, ctx->d_work_w, sCV, nc,
-                                          bits, ctx->d_work_x, nk, OLC_STAGE_ORTHO))) return st;
+    if ((st = ozaki_zgemm<double, double>(ctx, nv, nv, nc, scv, sCV, nc, true, bits, ocv, sCV, nc, bits, ctx->d_work_x,
+                                          nk, OLC_STAGE_ORTHO))) return st;
   }
   PackArgs a;
   a.vv = vv;
   a.X = ctx->d_work_x;
+  a.Y = Y;
   a.add = add;
   a.packed = packed;
   a.full = full;
@@ -252,13 +302,48 @@ int ortho_pack_ex(olc_context* ctx, bool is_overlap, const double* vv, const dou
   const size_t nt = (nv + kPackTile - 1) / kPackTile;
   StageScope scope(ctx, OLC_STAGE_ORTHO);
   ortho_pack_kernel<<<(int)std::min<size_t>(nt * (nt + 1) / 2 * nk, 152 * 32), 256, 0, ctx->stream>>>(a);
+  if (Y) cudaFreeAsync(Y, ctx->stream);
   return cuda_check(cudaGetLastError(), "ortho_pack_kernel");
+}
+
+// The same for blocks of a caller's own, synchronised.  Whether cc is Hermitian is
+// measured beside the product that takes it to be: the call waits for its end
+// anyway, and forms the general product in the rare case.  Hermitian: within 2^-44
+// of k's largest component, some ten times what the rounding of the integrals leaves
+// between the two triangles.
+int ortho_pack_blocks(olc_context* ctx, bool is_overlap, const double* vv, const double* cv, const double* cc,
+                      const double* scv, double* packed) {
+  const int nc = ctx->dims.core_dim, nk = ctx->dims.num_kpoints;
+  unsigned long long* dev = nullptr;
+  std::vector<double> asym(2 * (size_t)nk, 0.0);
+  int st;
+  if (nc) {
+    const size_t bytes = sizeof(unsigned long long) * 2 * (size_t)nk;
+    if ((st = cuda_check(ctx_malloc(ctx, (void**)&dev, bytes, ctx->stream), "malloc asymmetry"))) return st;
+    cudaMemsetAsync(dev, 0, bytes, ctx->stream);
+    const int nt = (nc + kPackTile - 1) / kPackTile;
+    StageScope scope(ctx, OLC_STAGE_ORTHO);
+    for (int k0 = 0; k0 < nk; k0 += 65535)
+      core_asymmetry_kernel<<<dim3(nt, nt, std::min(nk - k0, 65535)), 256, 0, ctx->stream>>>(
+          cc + 2 * (size_t)k0 * nc * nc, nc, dev + 2 * (size_t)k0);
+    cudaMemcpyAsync(asym.data(), dev, bytes, cudaMemcpyDeviceToHost, ctx->stream);
+    cudaFreeAsync(dev, ctx->stream);
+  }
+  st = ortho_pack_ex(ctx, is_overlap, vv, cv, cc, scv, packed, nullptr, nullptr, false);
+  if (!st) st = cuda_check(cudaStreamSynchronize(ctx->stream), "olc_ortho_pack sync");
+  if (st) return st;
+  for (int k = 0; k < nk; ++k)
+    if (!(asym[2 * k + 1] <= 0x1p-44 * asym[2 * k])) {
+      st = ortho_pack_ex(ctx, is_overlap, vv, cv, cc, scv, packed, nullptr, nullptr, true);
+      return st ? st : cuda_check(cudaStreamSynchronize(ctx->stream), "olc_ortho_pack sync");
+    }
+  return OLC_OK;
 }
 
 int ortho_pack(olc_context* ctx, bool is_overlap, double* vv, const double* cv, const double* cc,
                const double* scv, double* packed, double* full_out) {
   return ortho_pack_ex(ctx, is_overlap, vv, cv, cc, is_overlap ? cv : scv, packed, full_out,
-                       nullptr);
+                       nullptr, false);
 }
 
 int assemble_packed(olc_context* ctx, const double* const* terms, const double* coeffs, int nterm,
@@ -526,7 +611,7 @@ int scf_prepare(olc_context* ctx, int precision, int form) {
   if ((st = run_primitives(ctx, OLC_OP_OVERLAP, 0, nullptr, OLC_PREC_FP64, false))) return st;
   if ((st = run_contract_bloch(ctx, ctx->d_work_vv, nc ? ctx->d_scv : nullptr, ctx->d_work_cc))) return st;
   if ((st = ortho_pack_ex(ctx, true, ctx->d_work_vv, ctx->d_scv, ctx->d_work_cc, ctx->d_scv,
-                          nullptr, ctx->d_chol, nullptr))) return st;
+                          nullptr, ctx->d_chol, nullptr, false))) return st;
   count_launch();
   hermitize_kernel<<<grid_for(nn * nk), 256, 0, ctx->stream>>>(ctx->d_chol, nv, nk);
   const int nfix = 2 + ctx->rel;          // NP, KE (, MV) ahead of the V_j
@@ -540,7 +625,7 @@ int scf_prepare(olc_context* ctx, int precision, int form) {
       if ((st = run_primitives(ctx, op, t < nfix ? 0 : t - nfix, nullptr, OLC_PREC_FP64, false))) return st;
       if ((st = run_contract_bloch(ctx, ctx->d_work_vv, ctx->d_work_cv, ctx->d_work_cc))) return st;
       if ((st = ortho_pack_ex(ctx, false, ctx->d_work_vv, ctx->d_work_cv, ctx->d_work_cc,
-                              ctx->d_scv, ctx->d_terms + (size_t)t * plen2, nullptr, nullptr))) return st;
+                              ctx->d_scv, ctx->d_terms + (size_t)t * plen2, nullptr, nullptr, false))) return st;
     }
   } else {
     if (!ctx->d_h0 && (st = dalloc(ctx, &ctx->d_h0, 2 * nn * nk))) return st;
@@ -550,7 +635,7 @@ int scf_prepare(olc_context* ctx, int precision, int form) {
     if (ctx->rel && (st = run_primitives(ctx, OLC_OP_MASSVEL, 0, nullptr, OLC_PREC_FP64, true))) return st;
     if ((st = run_contract_bloch(ctx, ctx->d_work_vv, ctx->d_work_cv, ctx->d_work_cc))) return st;
     if ((st = ortho_pack_ex(ctx, false, ctx->d_work_vv, ctx->d_work_cv, ctx->d_work_cc, ctx->d_scv,
-                            nullptr, ctx->d_h0, nullptr))) return st;
+                            nullptr, ctx->d_h0, nullptr, false))) return st;
   }
   ctx->prepared = true;
   ctx->w32_valid = false;
@@ -713,7 +798,7 @@ int build_hamiltonian(olc_context* ctx, const double* coeffs, int precision, int
     if ((st = run_contract_bloch(ctx, ctx->d_work_vv, ctx->d_work_cv, ctx->d_work_cc))) return st;
     // H' = ortho(V) + H0, upper, then mirrored
     if ((st = ortho_pack_ex(ctx, false, ctx->d_work_vv, ctx->d_work_cv, ctx->d_work_cc, ctx->d_scv,
-                            nullptr, h, ctx->d_h0))) return st;
+                            nullptr, h, ctx->d_h0, false))) return st;
     StageScope scope(ctx, OLC_STAGE_ASSEMBLE);
     hermitize_kernel<<<grid_for(nn * nk), 256, 0, ctx->stream>>>(h, nv, nk);
   }
