@@ -105,6 +105,14 @@ int small_solver_max_n() {
   return v;
 }
 
+// The shared memory of the largest pencil, for every launch: a limit set to the
+// launch's own need could be lowered by another thread before it.
+static int allow_smem() {
+  return cuda_check(cudaFuncSetAttribute(small_hegv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)jac::smem_bytes(jac::kMaxN)),
+                    "smem attribute");
+}
+
 // s_full is overwritten with its Cholesky factors.
 int solve_small_batched(olc_context* ctx, const double* h_full, double* s_full, int n,
                         int num_states, double* eigenvalues, double* vectors, int32_t* info_host,
@@ -112,9 +120,7 @@ int solve_small_batched(olc_context* ctx, const double* h_full, double* s_full, 
   const int nk = ctx->dims.num_kpoints;
   const size_t smem = jac::smem_bytes(n);
   int st;
-  if ((st = cuda_check(cudaFuncSetAttribute(small_hegv_kernel,
-                                            cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
-                       "smem attribute"))) return st;
+  if ((st = allow_smem())) return st;
   int32_t* dinfo = nullptr;
   if ((st = cuda_check(ctx_malloc(ctx, (void**)&dinfo, sizeof(int32_t) * nk, ctx->stream), "malloc info"))) return st;
   StageScope scope(ctx, OLC_STAGE_SOLVE);
@@ -164,9 +170,7 @@ int launch_small_hegv_raw(cudaStream_t stream, const double* h_full, double* s_f
                           int32_t* info_dev) {
   const size_t smem = jac::smem_bytes(n);
   int st;
-  if ((st = cuda_check(cudaFuncSetAttribute(small_hegv_kernel,
-                                            cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
-                       "smem attribute"))) return st;
+  if ((st = allow_smem())) return st;
   count_launch();
   small_hegv_kernel<<<nk, threads_for(n), smem, stream>>>(h_full, s_full, n, num_states, 0, eigenvalues,
                                                     vectors, info_dev, nullptr);

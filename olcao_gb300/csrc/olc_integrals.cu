@@ -390,9 +390,9 @@ int run_contract_bloch(olc_context* ctx, double* vv, double* cv, double* cc) {
   ca.rows = 0;
   for (const DevType& t : ctx->htypes)
     ca.rows = std::max(ca.rows, t.nalpha * (t.lmax_alpha[0] + 1) * (t.lmax_alpha[0] + 1));
+  // at most 32 KB, with the static part below what every launch may have
+  static_assert(kContractCols * sizeof(double) * OLC_MAX_ALPHAS * nharm(kMaxL) <= 32 * 1024, "contraction table");
   const size_t csmem = sizeof(double) * kContractCols * (size_t)ca.rows;
-  if ((st = cuda_check(cudaFuncSetAttribute(contract_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)csmem),
-                       "contract smem"))) return st;
   {
     StageScope scope(ctx, OLC_STAGE_CONTRACT);
     const dim3 cgrid((unsigned)ntasks, (unsigned)((ctx->max_states + kContractCols - 1) / kContractCols));

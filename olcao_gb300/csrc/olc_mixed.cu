@@ -848,10 +848,14 @@ int solve_full_mixed(olc_context* ctx, const double* h, const double* s, int num
     int P = 1;
     while (P < n) P <<= 1;
     const size_t sortmem = (size_t)P * (sizeof(double) + sizeof(int));
+    // limits for the largest n (hetrd_max_n), whatever this call takes: a limit set to
+    // its own need could be lowered by another thread before its launch
+    constexpr int kMostSort = 16384 * (int)(sizeof(double) + sizeof(int));
+    if (sortmem > (size_t)kMostSort) return fail(OLC_ERR_UNSUPPORTED, "mixed solver: n above the sorting limit");
     if ((st = cuda_check(cudaFuncSetAttribute(cluster_sort_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                              (int)sortmem), "smem attribute"))) return st;
+                                              kMostSort), "smem attribute"))) return st;
     if ((st = cuda_check(cudaFuncSetAttribute(final_sort_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                              (int)sortmem), "smem attribute"))) return st;
+                                              kMostSort), "smem attribute"))) return st;
     if ((st = cuda_check(cudaMemsetAsync(L.counters, 0, 4 * sizeof(int), stream), "memset"))) return st;
     cluster_sort_kernel<<<nk, 1024, sortmem, stream>>>(Hh, n, L);
     if ((st = cuda_check(cudaMemsetAsync(reach, 0xff, 4ULL * n * nk, stream), "memset reach"))) return st;
@@ -865,7 +869,7 @@ int solve_full_mixed(olc_context* ctx, const double* h, const double* s, int num
     }
     const size_t formmem = (size_t)n * (sizeof(double) + sizeof(int));
     if ((st = cuda_check(cudaFuncSetAttribute(cluster_form_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                              (int)formmem), "smem attribute"))) return st;
+                                              kMostSort), "smem attribute"))) return st;
     // OLC_CLUSTER_GAP overrides the gap that separates clusters (Hartree)
     double gap = kClusterGap;
     if (const char* v = std::getenv("OLC_CLUSTER_GAP")) gap = std::atof(v);

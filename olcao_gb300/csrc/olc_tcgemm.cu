@@ -805,6 +805,9 @@ std::mutex g_err_mu;
 // K-blocks: the three-digit operand's six tiles live throughout, a window of
 // six of the other's); f32 mode rings of 6 of 16 KB and 4 of 32 KB.
 constexpr int kFixedSlots = 14;
+// the most a launch of either mode takes: the limit every launch sets (a limit set
+// to the launch's own need could be lowered by another thread before it)
+constexpr int kSmemMax = kFixedSlots * kTileBytesA + 512 + 1024;
 void plan_pairs(TcParams& p, int mode) {
   for (int i = 0; i < p.npairs; ++i) {
     TcPair& pr = p.pairs[i];
@@ -868,14 +871,14 @@ int launch(olc_context* ctx, int mode, const void* dA, const void* dB, int plane
   p.err = g_err;
   plan_pairs(p, mode);
   const dim3 grid((unsigned)(p.nmt * p.nnt), (unsigned)nb);
-  const int smem = smem_total(mode, p.slots_a, p.slots_b);
+  const int smem = smem_total(mode, p.slots_a, p.slots_b);     // at most kSmemMax
   if (mode == 0) {
-    if ((s = cuda_check(cudaFuncSetAttribute(tc_gemm_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem),
+    if ((s = cuda_check(cudaFuncSetAttribute(tc_gemm_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax),
                         "tc smem")))
       return s;
     tc_gemm_kernel<0><<<grid, kThreads, smem, st>>>(ta, tb, p);
   } else {
-    if ((s = cuda_check(cudaFuncSetAttribute(tc_gemm_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem),
+    if ((s = cuda_check(cudaFuncSetAttribute(tc_gemm_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax),
                         "tc smem")))
       return s;
     tc_gemm_kernel<1><<<grid, kThreads, smem, st>>>(ta, tb, p);
