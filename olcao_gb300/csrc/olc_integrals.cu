@@ -71,17 +71,24 @@ int launch_class(olc_context* ctx, cudaStream_t stream, int cls, const double* c
   return cuda_check(cudaGetLastError(), "primitive kernel launch");
 }
 
-// Side streams of the third-centre classes (created at first use).
+// Side streams of the third-centre classes (created at first use).  false: there are
+// none, the classes run one after the other; the error that said so is cleared, so
+// that it isn't taken for one of the launches that follow.
 constexpr int kSideStreams = 3;
 bool side_streams(olc_context* ctx) {
   if ((int)ctx->prim_streams.size() == kSideStreams) return true;
-  if (!ctx->prim_fork && cudaEventCreateWithFlags(&ctx->prim_fork, cudaEventDisableTiming) != cudaSuccess) return false;
+  if (!ctx->prim_fork && cudaEventCreateWithFlags(&ctx->prim_fork, cudaEventDisableTiming) != cudaSuccess) {
+    ctx->prim_fork = nullptr;
+    cudaGetLastError();
+    return false;
+  }
   while ((int)ctx->prim_streams.size() < kSideStreams) {
-    cudaStream_t st;
-    cudaEvent_t ev;
-    if (cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking) != cudaSuccess) return false;
-    if (cudaEventCreateWithFlags(&ev, cudaEventDisableTiming) != cudaSuccess) {
-      cudaStreamDestroy(st);
+    cudaStream_t st = nullptr;
+    cudaEvent_t ev = nullptr;
+    if (cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking) != cudaSuccess ||
+        cudaEventCreateWithFlags(&ev, cudaEventDisableTiming) != cudaSuccess) {
+      if (st) cudaStreamDestroy(st);
+      cudaGetLastError();
       return false;
     }
     ctx->prim_streams.push_back(st);
@@ -128,7 +135,6 @@ int run_primitives(olc_context* ctx, int op, int term, const double* coeffs, int
     st = cuda_check(cudaEventRecord(ctx->prim_fork, ctx->stream), "fork primitives");
     for (int q = 0; q < kSideStreams && !st; ++q)
       st = cuda_check(cudaStreamWaitEvent(ctx->prim_streams[q], ctx->prim_fork, 0), "fork primitives");
-    if (st) return st;
   }
   for (int c = 0; c < kNumClasses && !st; ++c) {
     const int cls = order[c];
