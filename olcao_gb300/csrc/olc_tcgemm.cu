@@ -31,9 +31,12 @@
 //    precision are not issued.  The result is acc scaled by
 //    2^(e_row + f_col + base): FP64 complex, no intermediate in global memory.
 //  * f32 mode (FP32-accurate products): x = x0 + x1 + x2 (three BF16 pieces
-//    of an FP32 value, 24 bits); the six pairs with weight >= 2^-16 of one
-//    K-block (384 products) accumulate in an FP32 TMEM accumulator, which is
-//    drained into register sums; C = alpha D + beta C.
+//    of an FP32 value, 24 bits); of the six pairs with weight >= 2^-16 the leading
+//    one has an accumulator of its own, where products of 16 bits lose little, and
+//    the five below share one (the tensor cores cut off what lies below the last
+//    place of the sum, a bias towards zero where small terms meet a large sum: all
+//    six in one accumulator were off by 3e-7 of like-signed sums, 1e-8 so).  Both
+//    collect kF32Span K-blocks and are drained into register sums; C = alpha D + beta C.
 //
 // GPU safety: every mbarrier wait is bounded by wall time (%globaltimer);
 // on expiry the thread records an error code, the other roles see it and
@@ -65,6 +68,7 @@ constexpr int kThreads = (kEpiWarps + 2) * 32;
 template <int MODE>
 constexpr int num_acc() { return MODE == 0 ? 4 : 2; }
 constexpr int kTmemCols = 512;
+constexpr int kF32Span = 4;        // K-blocks an accumulator of the f32 mode collects
 constexpr long long kWaitNs = 2000000000LL;   // 2 s per wait
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
@@ -201,8 +205,8 @@ inline int smem_total(int mode, int slots_a, int slots_b) {
 // for half of its pairs, the copies run at the 5.4 TB/s that all SMs together
 // reach, and what is left of the 34 pairs hides about a third of them.  In the
 // f32 mode the copies' latency at the K-steps' ends.  Measured: FP64-accurate
-// product of order 1248 1025 -> 818 us, FP32-accurate 78 -> 83 us (one partial
-// wave); a mixed pass over 64 matrices of order 832: FP64-accurate products
+// product of order 1248 1025 -> 818 us, FP32-accurate one with its slices 133 -> 125
+// us; a mixed pass over 64 matrices of order 832: FP64-accurate products
 // 22.7 -> 19 ms, FP32-accurate ones (as then formed) 18.5 -> 14.2 ms.
 // MODE 0 (fixed): BN = 128, four accumulators of 128 columns, int64 drains,
 //   FP64 complex output.  Epilogue warp w owns TMEM lanes 32 (w % 4) .. +31
@@ -259,6 +263,12 @@ __global__ void __launch_bounds__(kThreads, 1)
     const int lo = kb * BK, hi = lo + BK;
     return (lo < kmax && hi > kmin) || (lo < p.kp + kmax && hi > p.kp + kmin);
   };
+  // K-blocks that run, of which kF32Span share the accumulators (f32 mode)
+  int needed = p.kblocks;
+  if (tri) {
+    needed = 0;
+    for (int kb = 0; kb < p.kblocks; ++kb) needed += kb_needed(kb);
+  }
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < MAX_SLOTS; ++s) {
@@ -349,10 +359,16 @@ __global__ void __launch_bounds__(kThreads, 1)
     int buf = 0;                        // accumulator of the current group and its wrap-around parity
     uint32_t phacc = 1;
     TcPair pr = p.pairs[0];             // the next pair is read while this one is issued
+    int nth = 0;                        // K-steps run before this one
     for (int kb = 0; kb < p.kblocks && ok; ++kb) {
       if (!kb_needed(kb)) continue;
+      // f32 mode: first and last K-block of the accumulators
+      const bool opens = MODE == 0 || nth % kF32Span == 0;
+      const bool closes = MODE == 0 || nth % kF32Span == kF32Span - 1 || nth == needed - 1;
+      ++nth;
       for (int i = 0; i < p.npairs; ++i) {
-        const int flags = pr.flags;
+        const int flags = pr.flags & ~((opens ? 0 : kPairStart) | (closes ? 0 : kPairEnd));
+        const bool group_end = (pr.flags & kPairEnd) != 0;
         int sa = basea + pr.pa, sb = baseb + pr.pb;
         pr = p.pairs[i + 1 < p.npairs ? i + 1 : 0];
         uint32_t fa = pha, fb = phb;
@@ -380,8 +396,9 @@ __global__ void __launch_bounds__(kThreads, 1)
           if (flags & kPairLastB) umma_commit(&emptyB[sb]);
           if (flags & kPairEnd) umma_commit(&accfull[buf]);
         }
-        if (flags & kPairEnd) {
-          if (++buf == NACC) { buf = 0; phacc ^= 1u; }
+        if (group_end && ++buf == NACC) {
+          buf = 0;
+          if (closes) phacc ^= 1u;
         }
       }
       __syncwarp();
@@ -459,14 +476,13 @@ __global__ void __launch_bounds__(kThreads, 1)
         }
       }
     } else {
-      // every K-block's sums (384 products) are drained into register
+      // the sums of every kF32Span K-blocks are drained into register
       // accumulators with round-to-nearest adds, so that long sums of
       // like-signed terms are not left to the tensor core's accumulator alone
       float acc[CW];
 #pragma unroll
       for (int j = 0; j < CW; ++j) acc[j] = 0.f;
-      for (int kb = 0; kb < p.kblocks && ok; ++kb) {
-        if (!kb_needed(kb)) continue;
+      for (int kb = 0; kb < needed && ok; kb += kF32Span) {
         for (int i = 0; i < p.ngroups; ++i, ++g) {
           const int buf = g % NACC;
           ok = __all_sync(0xffffffffu, mbar_wait(&accfull[buf], (uint32_t)(g / NACC) & 1u, cta_err, p.err, 4));
@@ -1023,9 +1039,10 @@ int cgemm_f32(olc_context* ctx, int m, int n, int k, const float* A, long long s
   // the six piece pairs of weight 2^-16 and above, and with OLC_F32_PAIRS=9 the
   // three below as well: one plane of B (the wide tile) after the other, the
   // low-order one first, so that a slot of B is free again after its own pairs
-  // (the second index counts B's planes from the last: pairs (a, 2 - b))
-  static const int8_t six[6][2] = {{0, 0}, {0, 1}, {1, 1}, {0, 2}, {1, 2}, {2, 2}};
-  static const int8_t nine[9][2] = {{0, 0}, {1, 0}, {2, 0}, {0, 1}, {1, 1}, {2, 1}, {0, 2}, {1, 2}, {2, 2}};
+  // (the second index counts B's planes from the last: pairs (a, 2 - b)); the
+  // leading pair last, a group of its own
+  static const int8_t six[6][2] = {{0, 0}, {0, 1}, {1, 1}, {1, 2}, {2, 2}, {0, 2}};
+  static const int8_t nine[9][2] = {{0, 0}, {1, 0}, {2, 0}, {0, 1}, {1, 1}, {2, 1}, {1, 2}, {2, 2}, {0, 2}};
   TcParams plan{};
   const char* pv = std::getenv("OLC_F32_PAIRS");
   plan.npairs = pv && std::atoi(pv) == 9 ? 9 : 6;
@@ -1034,8 +1051,9 @@ int cgemm_f32(olc_context* ctx, int m, int n, int k, const float* A, long long s
     plan.pairs[i] = TcPair{q[0], q[1], 0};
   }
   plan.pairs[0].flags |= kPairStart;
-  plan.pairs[plan.npairs - 1].flags |= kPairEnd;
-  plan.ngroups = 1;
+  plan.pairs[plan.npairs - 2].flags |= kPairEnd;
+  plan.pairs[plan.npairs - 1].flags |= kPairStart | kPairEnd;
+  plan.ngroups = num_acc<1>();     // one accumulator each: a group's stays its own over K-blocks
   plan.kspan = 1;
   const size_t per_b = 2 * Kp * 3 * ((size_t)m + 2 * (size_t)n);
   const int chunk = (int)std::max<size_t>(1, std::min<size_t>(nb, (8ULL << 30) / std::max<size_t>(per_b, 1)));
