@@ -163,6 +163,7 @@ struct olc_context {
   double* d_work_x = nullptr;      // GEMM temporaries
   double* d_work_p = nullptr;
   double* d_work_w = nullptr;
+  unsigned long long* d_asym = nullptr;   // olc_ortho_pack: magnitudes of cc and cc - cc^H per k
   void* d_solver_work = nullptr;
   size_t solver_work_bytes = 0;
   // independent k-point solves run concurrently on sub-streams

@@ -314,22 +314,21 @@ int ortho_pack_ex(olc_context* ctx, bool is_overlap, const double* vv, const dou
 int ortho_pack_blocks(olc_context* ctx, bool is_overlap, const double* vv, const double* cv, const double* cc,
                       const double* scv, double* packed) {
   const int nc = ctx->dims.core_dim, nk = ctx->dims.num_kpoints;
-  unsigned long long* dev = nullptr;
   std::vector<double> asym(2 * (size_t)nk, 0.0);
+  const size_t bytes = sizeof(double) * asym.size();
   int st;
   if (nc) {
-    const size_t bytes = sizeof(unsigned long long) * 2 * (size_t)nk;
-    if ((st = cuda_check(ctx_malloc(ctx, (void**)&dev, bytes, ctx->stream), "malloc asymmetry"))) return st;
-    cudaMemsetAsync(dev, 0, bytes, ctx->stream);
+    if (!ctx->d_asym && (st = dalloc(ctx, &ctx->d_asym, asym.size()))) return st;
+    cudaMemsetAsync(ctx->d_asym, 0, bytes, ctx->stream);
     const int nt = (nc + kPackTile - 1) / kPackTile;
     StageScope scope(ctx, OLC_STAGE_ORTHO);
     for (int k0 = 0; k0 < nk; k0 += 65535)
       core_asymmetry_kernel<<<dim3(nt, nt, std::min(nk - k0, 65535)), 256, 0, ctx->stream>>>(
-          cc + 2 * (size_t)k0 * nc * nc, nc, dev + 2 * (size_t)k0);
-    cudaMemcpyAsync(asym.data(), dev, bytes, cudaMemcpyDeviceToHost, ctx->stream);
-    cudaFreeAsync(dev, ctx->stream);
+          cc + 2 * (size_t)k0 * nc * nc, nc, ctx->d_asym + 2 * (size_t)k0);
   }
   st = ortho_pack_ex(ctx, is_overlap, vv, cv, cc, scv, packed, nullptr, nullptr, false);
+  // behind the product, as a copy to the host's own memory holds the caller up
+  if (!st && nc) st = cuda_check(cudaMemcpyAsync(asym.data(), ctx->d_asym, bytes, cudaMemcpyDeviceToHost, ctx->stream), "copy asymmetry");
   if (!st) st = cuda_check(cudaStreamSynchronize(ctx->stream), "olc_ortho_pack sync");
   if (st) return st;
   for (int k = 0; k < nk; ++k)
