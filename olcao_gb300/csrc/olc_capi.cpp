@@ -141,6 +141,7 @@ int olc_destroy(olc_context_t* ctx) {
   drain_profile(ctx);
   for (cudaEvent_t e : ctx->prof_pool) cudaEventDestroy(e);
   for (void* p : ctx->allocations) cudaFree(p);
+  if (ctx->h_asym) cudaFreeHost(ctx->h_asym);
   if (ctx->d_solver_work) cudaFree(ctx->d_solver_work);
   for (size_t i = 0; i < ctx->sub_streams.size(); ++i) {
     cudaStreamSynchronize(ctx->sub_streams[i]);

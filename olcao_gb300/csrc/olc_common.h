@@ -163,7 +163,8 @@ struct olc_context {
   double* d_work_x = nullptr;      // GEMM temporaries
   double* d_work_p = nullptr;
   double* d_work_w = nullptr;
-  unsigned long long* d_asym = nullptr;   // olc_ortho_pack: magnitudes of cc and cc - cc^H per k
+  unsigned long long* d_asym = nullptr;   // olc_ortho_pack: magnitudes of cc and cc - cc^H per k,
+  double* h_asym = nullptr;               // and their page-locked copy
   void* d_solver_work = nullptr;
   size_t solver_work_bytes = 0;
   // independent k-point solves run concurrently on sub-streams
@@ -275,6 +276,7 @@ int primitive_batch_device(int kind, int n, const double* in, const int32_t* lma
                            double* out);
 
 // dense stages (olc_linalg.cu)
+bool side_streams(olc_context* ctx);    // prim_streams, prim_fork (olc_integrals.cu)
 int ortho_pack(olc_context* ctx, bool is_overlap, double* vv, const double* cv,
                const double* cc, const double* scv, double* packed, double* full_out);
 int assemble_packed(olc_context* ctx, const double* const* terms, const double* coeffs,

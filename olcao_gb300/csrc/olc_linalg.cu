@@ -49,6 +49,7 @@ constexpr int kPackTile = 32;
 // block finds its tile once in FP32; an FP64 square root per element (1/64 of
 // the FP32 rate) and the strided mirror reads took 2.1 ms for 19 operators of
 // order 832 at 8 k-points, this form 0.78 ms.
+template <bool GENERAL>     // with Y
 __global__ void __launch_bounds__(256) ortho_pack_kernel(PackArgs a) {
   __shared__ double2 mirror[kPackTile][kPackTile + 1];
   const int nt = (a.nv + kPackTile - 1) / kPackTile;
@@ -83,7 +84,7 @@ __global__ void __launch_bounds__(256) ortho_pack_kernel(PackArgs a) {
         v.x -= x.x + m.x;
         v.y -= x.y - m.y;
         if (i == j) v.y = 0.0;
-        if (Y) {
+        if (GENERAL) {
           v.x += Y[off].x;
           v.y += Y[off].y;
         }
@@ -134,36 +135,56 @@ __global__ void __launch_bounds__(256) core_fold_kernel(const double2* __restric
 
 // Largest magnitudes of a component of O_cc and of O_cc - O_cc^H per k (as the bits
 // of doubles, which order like the non-negative numbers and NaN above them):
-// out[2 k], out[2 k + 1], zero on entry.  32 x 32 tiles of the lower triangle.
+// out[2 k], out[2 k + 1], zero on entry; one tile a k alone writes them as they are.
+// 32 x 32 tiles of the lower triangle.
 __global__ void __launch_bounds__(256) core_asymmetry_kernel(const double* __restrict__ cc, int nc,
                                                              unsigned long long* __restrict__ out) {
+  __shared__ unsigned long long most[2];
   __shared__ double2 mirror[kPackTile][kPackTile + 1];
   const int r0 = blockIdx.x * kPackTile, c0 = blockIdx.y * kPackTile;
   if (c0 > r0) return;
   const double* a = cc + 2 * (size_t)blockIdx.z * nc * nc;       // the caller's: any 8-byte address
   const int lane = threadIdx.x & 31, row0 = threadIdx.x >> 5;
-  for (int q = row0; q < kPackTile; q += 8)
-    if (r0 + q < nc && c0 + lane < nc) {
-      const size_t at = 2 * ((size_t)(r0 + q) * nc + c0 + lane);                // (row c0 + lane, column r0 + q)
-      mirror[q][lane] = make_double2(a[at], a[at + 1]);
+  if (threadIdx.x < 2) most[threadIdx.x] = 0;
+  constexpr int kPer = kPackTile / 8;
+  double2 x[kPer];               // (row r0 + lane, column c0 + q): both tiles' loads in flight together
+#pragma unroll
+  for (int j = 0; j < kPer; ++j) {
+    const int q = row0 + 8 * j;
+    x[j] = make_double2(0.0, 0.0);
+    if (c0 + q < nc && r0 + lane < nc) {
+      const double* p = a + 2 * ((size_t)(c0 + q) * nc + r0 + lane);
+      x[j] = make_double2(p[0], p[1]);
     }
+    if (r0 + q < nc && c0 + lane < nc) {
+      const double* p = a + 2 * ((size_t)(r0 + q) * nc + c0 + lane);            // (row c0 + lane, column r0 + q)
+      mirror[q][lane] = make_double2(p[0], p[1]);
+    }
+  }
   __syncthreads();
   unsigned long long big = 0, off = 0;
-  const auto bits = [](double x) { return (unsigned long long)__double_as_longlong(fabs(x)); };
-  for (int q = row0; q < kPackTile; q += 8)
+  const auto bits = [](double v) { return (unsigned long long)__double_as_longlong(fabs(v)); };
+#pragma unroll
+  for (int j = 0; j < kPer; ++j) {
+    const int q = row0 + 8 * j;
     if (c0 + q < nc && r0 + lane < nc) {
-      const size_t at = 2 * ((size_t)(c0 + q) * nc + r0 + lane);
-      const double2 x = make_double2(a[at], a[at + 1]), m = mirror[lane][q];
-      big = max(max(big, max(bits(x.x), bits(x.y))), max(bits(m.x), bits(m.y)));
-      off = max(off, max(bits(x.x - m.x), bits(x.y + m.y)));
+      const double2 m = mirror[lane][q];
+      big = max(max(big, max(bits(x[j].x), bits(x[j].y))), max(bits(m.x), bits(m.y)));
+      off = max(off, max(bits(x[j].x - m.x), bits(x[j].y + m.y)));
     }
+  }
   for (int o = 16; o; o >>= 1) {
     big = max(big, __shfl_xor_sync(0xffffffffu, big, o));
     off = max(off, __shfl_xor_sync(0xffffffffu, off, o));
   }
   if (lane == 0) {
-    atomicMax(&out[2 * blockIdx.z], big);
-    atomicMax(&out[2 * blockIdx.z + 1], off);
+    atomicMax(&most[0], big);
+    atomicMax(&most[1], off);
+  }
+  __syncthreads();
+  if (threadIdx.x < 2) {
+    if (gridDim.x == 1) out[2 * blockIdx.z + threadIdx.x] = most[threadIdx.x];
+    else atomicMax(&out[2 * blockIdx.z + threadIdx.x], most[threadIdx.x]);
   }
 }
 
@@ -301,38 +322,46 @@ int ortho_pack_ex(olc_context* ctx, bool is_overlap, const double* vv, const dou
   a.nc = nc;
   const size_t nt = (nv + kPackTile - 1) / kPackTile;
   StageScope scope(ctx, OLC_STAGE_ORTHO);
-  ortho_pack_kernel<<<(int)std::min<size_t>(nt * (nt + 1) / 2 * nk, 152 * 32), 256, 0, ctx->stream>>>(a);
+  const auto kern = Y ? ortho_pack_kernel<true> : ortho_pack_kernel<false>;
+  kern<<<(int)std::min<size_t>(nt * (nt + 1) / 2 * nk, 152 * 32), 256, 0, ctx->stream>>>(a);
   if (Y) cudaFreeAsync(Y, ctx->stream);
   return cuda_check(cudaGetLastError(), "ortho_pack_kernel");
 }
 
 // The same for blocks of a caller's own, synchronised.  Whether cc is Hermitian is
-// measured beside the product that takes it to be: the call waits for its end
-// anyway, and forms the general product in the rare case.  Hermitian: within 2^-44
-// of k's largest component, some ten times what the rounding of the integrals leaves
-// between the two triangles.
+// measured beside the product that takes it to be, and the rare other case is formed
+// again in general.  Hermitian: within 2^-44 of k's largest component, some ten times
+// what the rounding of the integrals leaves between the two triangles.  One tile a k
+// goes behind the product and writes to the host's memory; more of them go on a side
+// stream (Si64: 16 us that would else add to the product's 1.1 ms).
 int ortho_pack_blocks(olc_context* ctx, bool is_overlap, const double* vv, const double* cv, const double* cc,
                       const double* scv, double* packed) {
-  const int nc = ctx->dims.core_dim, nk = ctx->dims.num_kpoints;
-  std::vector<double> asym(2 * (size_t)nk, 0.0);
-  const size_t bytes = sizeof(double) * asym.size();
+  const int nc = ctx->dims.core_dim, nk = ctx->dims.num_kpoints, nt = (nc + kPackTile - 1) / kPackTile;
+  const size_t bytes = sizeof(double) * 2 * (size_t)nk;
+  const bool side = nt > 1 && side_streams(ctx);
+  const cudaStream_t on = side ? ctx->prim_streams[0] : ctx->stream;
   int st;
-  if (nc) {
-    if (!ctx->d_asym && (st = dalloc(ctx, &ctx->d_asym, asym.size()))) return st;
-    cudaMemsetAsync(ctx->d_asym, 0, bytes, ctx->stream);
-    const int nt = (nc + kPackTile - 1) / kPackTile;
-    StageScope scope(ctx, OLC_STAGE_ORTHO);
-    for (int k0 = 0; k0 < nk; k0 += 65535)
-      core_asymmetry_kernel<<<dim3(nt, nt, std::min(nk - k0, 65535)), 256, 0, ctx->stream>>>(
-          cc + 2 * (size_t)k0 * nc * nc, nc, ctx->d_asym + 2 * (size_t)k0);
+  if (nc && !ctx->h_asym) {
+    if ((st = dalloc(ctx, &ctx->d_asym, 2 * (size_t)nk))) return st;
+    if ((st = cuda_check(cudaMallocHost((void**)&ctx->h_asym, bytes), "malloc asymmetry"))) return st;
   }
-  st = ortho_pack_ex(ctx, is_overlap, vv, cv, cc, scv, packed, nullptr, nullptr, false);
-  // behind the product, as a copy to the host's own memory holds the caller up
-  if (!st && nc) st = cuda_check(cudaMemcpyAsync(asym.data(), ctx->d_asym, bytes, cudaMemcpyDeviceToHost, ctx->stream), "copy asymmetry");
-  if (!st) st = cuda_check(cudaStreamSynchronize(ctx->stream), "olc_ortho_pack sync");
-  if (st) return st;
+  if (side && (st = cuda_check(cudaEventRecord(ctx->prim_fork, ctx->stream), "fork asymmetry"))) return st;
+  if ((st = ortho_pack_ex(ctx, is_overlap, vv, cv, cc, scv, packed, nullptr, nullptr, false))) return st;
+  if (nc) {
+    unsigned long long* out = nt > 1 ? ctx->d_asym : reinterpret_cast<unsigned long long*>(ctx->h_asym);
+    if (side && (st = cuda_check(cudaStreamWaitEvent(on, ctx->prim_fork, 0), "fork asymmetry"))) return st;
+    if (nt > 1) cudaMemsetAsync(out, 0, bytes, on);
+    for (int k0 = 0; k0 < nk; k0 += 65535) {
+      count_launch();
+      core_asymmetry_kernel<<<dim3(nt, nt, std::min(nk - k0, 65535)), 256, 0, on>>>(cc + 2 * (size_t)k0 * nc * nc, nc,
+                                                                                    out + 2 * (size_t)k0);
+    }
+    if (nt > 1) cudaMemcpyAsync(ctx->h_asym, out, bytes, cudaMemcpyDeviceToHost, on);
+    if (side && (st = cuda_check(cudaStreamSynchronize(on), "olc_ortho_pack sync"))) return st;
+  }
+  if ((st = cuda_check(cudaStreamSynchronize(ctx->stream), "olc_ortho_pack sync")) || !nc) return st;
   for (int k = 0; k < nk; ++k)
-    if (!(asym[2 * k + 1] <= 0x1p-44 * asym[2 * k])) {
+    if (!(ctx->h_asym[2 * k + 1] <= 0x1p-44 * ctx->h_asym[2 * k])) {
       st = ortho_pack_ex(ctx, is_overlap, vv, cv, cc, scv, packed, nullptr, nullptr, true);
       return st ? st : cuda_check(cudaStreamSynchronize(ctx->stream), "olc_ortho_pack sync");
     }

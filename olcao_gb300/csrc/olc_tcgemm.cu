@@ -265,7 +265,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   };
   // K-blocks that run, of which kF32Span share the accumulators (f32 mode)
   int needed = p.kblocks;
-  if (tri) {
+  if (MODE == 1 && tri) {
     needed = 0;
     for (int kb = 0; kb < p.kblocks; ++kb) needed += kb_needed(kb);
   }
@@ -365,10 +365,10 @@ __global__ void __launch_bounds__(kThreads, 1)
       // f32 mode: first and last K-block of the accumulators
       const bool opens = MODE == 0 || nth % kF32Span == 0;
       const bool closes = MODE == 0 || nth % kF32Span == kF32Span - 1 || nth == needed - 1;
-      ++nth;
+      if (MODE == 1) ++nth;
       for (int i = 0; i < p.npairs; ++i) {
-        const int flags = pr.flags & ~((opens ? 0 : kPairStart) | (closes ? 0 : kPairEnd));
-        const bool group_end = (pr.flags & kPairEnd) != 0;
+        const int all = pr.flags;
+        const int flags = MODE == 0 ? all : all & ~((opens ? 0 : kPairStart) | (closes ? 0 : kPairEnd));
         int sa = basea + pr.pa, sb = baseb + pr.pb;
         pr = p.pairs[i + 1 < p.npairs ? i + 1 : 0];
         uint32_t fa = pha, fb = phb;
@@ -396,9 +396,11 @@ __global__ void __launch_bounds__(kThreads, 1)
           if (flags & kPairLastB) umma_commit(&emptyB[sb]);
           if (flags & kPairEnd) umma_commit(&accfull[buf]);
         }
-        if (group_end && ++buf == NACC) {
-          buf = 0;
-          if (closes) phacc ^= 1u;
+        if (all & kPairEnd) {
+          if (++buf == NACC) {
+            buf = 0;
+            if (MODE == 0 || closes) phacc ^= 1u;
+          }
         }
       }
       __syncwarp();
@@ -454,10 +456,9 @@ __global__ void __launch_bounds__(kThreads, 1)
           } else {
             // low-order digit groups: rounded to the accumulator's unit (a
             // plain arithmetic shift would floor, a bias of half a unit per
-            // drain that adds up over long K).  |v| < 2^24, so that a shift by 26
-            // and more gives 0, and one past 30 (K of a million) may stop there
-            const int right = min(-sh, 30), half = 1 << (right - 1);
-            drain([right, half](long long& x, int v) { x += (v + half) >> right; });
+            // drain that adds up over long K)
+            const int half = 1 << (-sh - 1);
+            drain([sh, half](long long& x, int v) { x += (v + half) >> (-sh); });
           }
         }
       }
@@ -978,7 +979,9 @@ int zgemm_fixed(olc_context* ctx, int m, int n, int k, const TA* A, long long sA
     if (plan.npairs == first) continue;
     plan.pairs[first].flags |= kPairStart;
     plan.pairs[plan.npairs - 1].flags |= kPairEnd;
-    plan.shift[plan.ngroups++] = (int16_t)(kBeta * (T - d) - L);
+    // a group's sum is below 2^24, so that a shift to the right by 26 and more gives
+    // 0, and one past 30 (K of a million) may stop there: half a unit fits 32 bits
+    plan.shift[plan.ngroups++] = (int16_t)std::max(kBeta * (T - d) - L, -30);
   }
   // batch chunk: digit planes below ~8 GB
   const size_t per_b = 2 * Kp * ((size_t)na * m + (size_t)nbd * 2 * n);
