@@ -79,8 +79,8 @@ struct SysView {
   // [atom][potential type], ordered by shells of |C' - A| within a group:
   // every image a third-centre sum of an alpha pair on A can reach
   const int32_t* img_start;          // [natoms*num_pot_types + 1]
-  const double4_16a* img_d;              // C' - A (x, y, z, 0)
-  const float4* img_hi;              // C' - A rounded; w: below |C' - A|, its shell
+  const double4_16a* img_d;          // C' - A; w: below |C' - A|, its shell's inner radius
+  const float4* img_hi;              // both rounded
   const float4* img_lo;              // the rounding's remainder
   const double* elem_alpha;          // [nelem*OLC_MAX_ALPHAS]
   const double* elem_nuc_alpha;      // [nelem]

@@ -13,8 +13,10 @@
 //                          the reference's diagonal/mode walk enumerates because
 //                          the exponents ascend)
 #include <algorithm>
+#include <array>
 #include <cmath>
 #include <cstring>
+#include <functional>
 
 #include "olc_common.h"
 
@@ -123,13 +125,27 @@ int upload(olc_context* ctx, T** dst, const std::vector<T>& src) {
 // that radius, at the smallest exponents, bounds the list.
 // Within a group the images are ordered by distance shells of rad / kShells
 // (a counting sort; the kernels stop at the first shell past their reach).
+// Bound by writing the list, 32 bytes an image: its FP32 pairs are formed on the
+// device, and the list has its room from the start (113400 images of the 216-atom
+// silicon cell: olc_create 18.9 ms with 64 bytes an image in growing arrays and each
+// task's items taken from the type pair's full list, 9.3 ms so).
 constexpr int kShells = 64;
 
 struct Images {
   std::vector<int32_t> start;
-  std::vector<double4_16a> d;
-  std::vector<float4> hi, lo;
+  std::vector<double4_16a> d;         // w: below |C' - A|, the shell's inner radius
 };
+
+// The FP32 pairs of the images' vectors (SysView::img_hi, img_lo).
+__global__ void image_pairs_kernel(const double4_16a* __restrict__ d, size_t n, float4* __restrict__ hi,
+                                   float4* __restrict__ lo) {
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
+    const double4_16a x = d[i];
+    const float4 h = make_float4((float)x.x, (float)x.y, (float)x.z, (float)x.w);
+    hi[i] = h;
+    lo[i] = make_float4((float)(x.x - h.x), (float)(x.y - h.y), (float)(x.z - h.z), 0.f);
+  }
+}
 
 void make_images(const Lattice& lat, const olc_context* ctx, const std::vector<int32_t>& siteType,
                  const std::vector<double>& sitePos, const double* potPos, const std::vector<double>& elemAlpha,
@@ -144,7 +160,9 @@ void make_images(const Lattice& lat, const olc_context* ctx, const std::vector<i
   for (int l = 0; l < 3; ++l)
     plane[l] = std::sqrt(lat.inv[l][0] * lat.inv[l][0] + lat.inv[l][1] * lat.inv[l][1] + lat.inv[l][2] * lat.inv[l][2]);
   im.start.push_back(0);
-  std::vector<double4_16a> found;     // w = |C' - A|^2
+  std::vector<double4_16a> found;
+  std::vector<uint8_t> shell;         // of each one found
+  std::vector<int32_t> order;
   for (int i = 0; i < ns; ++i) {
     const DevType& t1 = ctx->htypes[siteType[i]];
     const double a1 = elemAlpha[(size_t)t1.element * OLC_MAX_ALPHAS];
@@ -160,8 +178,9 @@ void make_images(const Lattice& lat, const olc_context* ctx, const std::vector<i
         rad = std::sqrt(maxSep) + std::sqrt(T * (1.0 / minAlpha + 1.0 / a3));
       rad *= 1.0 + 1e-6;
       if (!(a3 > 0.0) || !(rad < 1e6)) rad = std::sqrt(lat.cells.back());
-      const double rad2 = rad * rad;
+      const double rad2 = rad * rad, per = kShells / rad;
       found.clear();
+      shell.clear();
       for (int m = 0; m < pt.multiplicity; ++m) {
         double v[3];
         int lo[3], hi[3];
@@ -184,28 +203,25 @@ void make_images(const Lattice& lat, const olc_context* ctx, const std::vector<i
                 x[c] = v[c] + (y[c] + lat.rv[2][c] * n2);
                 d2 += x[c] * x[c];
               }
-              if (d2 <= rad2) found.push_back(make_double4_16a(x[0], x[1], x[2], d2));
+              if (d2 <= rad2) {
+                found.push_back(make_double4_16a(x[0], x[1], x[2], 0.0));
+                shell.push_back((uint8_t)std::min(kShells - 1, (int)(per * std::sqrt(d2))));
+              }
             }
           }
       }
-      auto shell = [&](double d2) { return std::min(kShells - 1, (int)(kShells * std::sqrt(d2) / rad)); };
       int32_t at[kShells + 1] = {};
-      for (const auto& x : found) ++at[shell(x.w) + 1];
+      for (uint8_t q : shell) ++at[q + 1];
       for (int q = 0; q < kShells; ++q) at[q + 1] += at[q];
-      const size_t base = im.d.size();
-      im.d.resize(base + found.size());
-      im.hi.resize(base + found.size());
-      im.lo.resize(base + found.size());
-      for (const auto& x : found) {
-        const int q = shell(x.w);
-        const size_t o = base + at[q]++;
-        const float4 h = make_float4((float)x.x, (float)x.y, (float)x.z, (float)(0.999999 * rad / kShells * q));
-        im.d[o] = x;
-        im.hi[o] = h;
-        im.lo[o] = make_float4((float)(x.x - h.x), (float)(x.y - h.y), (float)(x.z - h.z), 0.f);
+      order.resize(found.size());
+      for (size_t o = 0; o < found.size(); ++o) order[at[shell[o]]++] = (int32_t)o;
+      for (int32_t o : order) {
+        im.d.push_back(found[o]);
+        im.d.back().w = 0.999999 * rad / kShells * shell[o];
       }
       im.start.push_back((int32_t)im.d.size());
     }
+    if (i == 0) im.d.reserve((im.d.size() + im.d.size() / 8) * ns);   // the other atoms' lists are much alike
   }
 }
 
@@ -453,16 +469,40 @@ int build_system(olc_context* ctx, const olc_system_t* s) {
       }
       std::stable_sort(tp.begin(), tp.end(), [](const AlphaPair& p, const AlphaPair& q) { return p.sum < q.sum; });
     }
+  // Tasks between the same two of a type pair's radii have the same items: each such
+  // list is made once, by class, when the first of its tasks asks for it.
+  struct Reach {
+    std::vector<double> radius;                                   // descending, each once
+    std::vector<std::array<std::vector<int32_t>, kNumClasses>> ab;   // of the pairs with dist >= radius[q]
+  };
+  std::vector<Reach> reach(typePairs.size());
+  for (size_t x = 0; x < typePairs.size(); ++x) {
+    Reach& r = reach[x];
+    for (const AlphaPair& e : typePairs[x]) r.radius.push_back(e.dist);
+    std::sort(r.radius.begin(), r.radius.end(), std::greater<double>());
+    r.radius.erase(std::unique(r.radius.begin(), r.radius.end()), r.radius.end());
+    r.ab.resize(r.radius.size());
+  }
   std::vector<int32_t> itTask[kNumClasses], itAB[kNumClasses], itStart[kNumClasses];
   for (int c = 0; c < kNumClasses; ++c) itStart[c].assign(ntasks + 1, 0);
   for (int q = 0; q < ntasks; ++q) {
     const DevTask& tk = ctx->htasks[q];
     const DevPair& p = ctx->hpairs[tk.pair];
     for (int c = 0; c < kNumClasses; ++c) itStart[c][q] = (int32_t)itTask[c].size();
-    for (const AlphaPair& e : typePairs[(size_t)siteType[p.i] * s->num_atom_types + siteType[p.j]]) {
-      if (e.dist < tk.sep) continue;
-      itTask[e.cls].push_back(q);
-      itAB[e.cls].push_back(e.ab);
+    const size_t x = (size_t)siteType[p.i] * s->num_atom_types + siteType[p.j];
+    Reach& r = reach[x];
+    const size_t in = std::partition_point(r.radius.begin(), r.radius.end(),
+                                           [&](double d) { return !(d < tk.sep); }) - r.radius.begin();
+    if (in == 0) continue;
+    auto& list = r.ab[in - 1];
+    bool made = false;
+    for (const auto& l : list) made = made || !l.empty();
+    if (!made)
+      for (const AlphaPair& e : typePairs[x])
+        if (e.dist >= r.radius[in - 1]) list[e.cls].push_back(e.ab);
+    for (int c = 0; c < kNumClasses; ++c) {
+      itTask[c].insert(itTask[c].end(), list[c].size(), q);
+      itAB[c].insert(itAB[c].end(), list[c].begin(), list[c].end());
     }
   }
   for (int c = 0; c < kNumClasses; ++c) itStart[c][ntasks] = (int32_t)itTask[c].size();
@@ -518,15 +558,19 @@ int build_system(olc_context* ctx, const olc_system_t* s) {
     Images im;
     make_images(lat, ctx, siteType, sitePos, s->pot_site_pos, elemAlpha, elemPot, elemNuc, T, im);
     double4_16a* d4;
-    float4* f4;
+    float4 *hi = nullptr, *lo = nullptr;
     if ((st = upload(ctx, &dst, im.start))) return st;
     v.img_start = dst;
     if ((st = upload(ctx, &d4, im.d))) return st;
     v.img_d = d4;
-    if ((st = upload(ctx, &f4, im.hi))) return st;
-    v.img_hi = f4;
-    if ((st = upload(ctx, &f4, im.lo))) return st;
-    v.img_lo = f4;
+    if (const size_t n = im.d.size()) {
+      if ((st = dalloc(ctx, &hi, n)) || (st = dalloc(ctx, &lo, n))) return st;
+      count_launch();
+      image_pairs_kernel<<<(int)std::min<size_t>((n + 255) / 256, 152 * 8), 256, 0, ctx->stream>>>(d4, n, hi, lo);
+      if ((st = cuda_check(cudaGetLastError(), "image_pairs_kernel"))) return st;
+    }
+    v.img_hi = hi;
+    v.img_lo = lo;
   }
   if ((st = upload(ctx, &dd, elemAlpha))) return st;
   v.elem_alpha = dd;
