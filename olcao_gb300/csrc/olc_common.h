@@ -72,9 +72,6 @@ struct SysView {
   int32_t ncells;
   const DevPotType* pot_types;
   int32_t num_pot_types;
-  const double* pot_site_pos;        // [3*npotsites]
-  const int32_t* pot_site_type;
-  int32_t num_pot_sites;
   // images C' = C + T of the potential sites around each atom A, grouped by
   // [atom][potential type], ordered by shells of |C' - A| within a group:
   // every image a third-centre sum of an alpha pair on A can reach
@@ -85,8 +82,6 @@ struct SysView {
   const double* elem_alpha;          // [nelem*OLC_MAX_ALPHAS]
   const double* elem_nuc_alpha;      // [nelem]
   const double* elem_pot_alpha;      // [nelem*OLC_MAX_POT_ALPHAS]
-  double inv_real[9];                // invRealVectors(i, xyz) row-major [abc][xyz]
-  double real_vec[9];                // [abc][xyz]
   double log_thresh;                 // T = -ln(BASIS_FN thresh)
   int32_t vale_dim, core_dim, nk;
   const double* kxyz;                // [3*nk]

@@ -547,13 +547,6 @@ int build_system(olc_context* ctx, const olc_system_t* s) {
   if ((st = upload(ctx, &dPots, ctx->hpots))) return st;
   v.pot_types = dPots;
   v.num_pot_types = npt;
-  std::vector<double> potPos(s->pot_site_pos, s->pot_site_pos + 3 * s->num_pot_sites);
-  std::vector<int32_t> potType(s->pot_site_type, s->pot_site_type + s->num_pot_sites);
-  if ((st = upload(ctx, &dd, potPos))) return st;
-  v.pot_site_pos = dd;
-  if ((st = upload(ctx, &dst, potType))) return st;
-  v.pot_site_type = dst;
-  v.num_pot_sites = s->num_pot_sites;
   {
     Images im;
     make_images(lat, ctx, siteType, sitePos, s->pot_site_pos, elemAlpha, elemPot, elemNuc, T, im);
@@ -578,11 +571,6 @@ int build_system(olc_context* ctx, const olc_system_t* s) {
   v.elem_nuc_alpha = dd;
   if ((st = upload(ctx, &dd, elemPot))) return st;
   v.elem_pot_alpha = dd;
-  for (int i = 0; i < 3; ++i)
-    for (int c = 0; c < 3; ++c) {
-      v.inv_real[i * 3 + c] = lat.inv[i][c];
-      v.real_vec[i * 3 + c] = lat.rv[i][c];
-    }
   v.log_thresh = T;
   v.vale_dim = valeDim;
   v.core_dim = coreDim;
