@@ -168,7 +168,7 @@ __global__ void __launch_bounds__(kThirdThreads) third_centre_kernel(SysView v, 
     d2ab += ab * ab;
     ps2 += PS[c] * PS[c];
   }
-  const double expAB = exp(-(g.a1 * g.a2 * iz) * d2ab);
+  const double expAB = exp(-ratio(g.a1 * g.a2, z, iz) * d2ab);
   const float psf[3] = {(float)PS[0], (float)PS[1], (float)PS[2]};
   const float ap = (float)sqrt(ps2);
   float pah[3], pal[3];
@@ -204,7 +204,7 @@ __global__ void __launch_bounds__(kThirdThreads) third_centre_kernel(SysView v, 
                                              : v.elem_pot_alpha[pt.element * OLC_MAX_POT_ALPHAS + j];
       const double tad = frac * (T * (al + ak + an) * izs / an);
       const double a3 = OP == OLC_OP_NUCLEAR ? pt.nuc_alpha : pt.alphas[j];
-      const double z3 = z + a3, iz3 = 1.0 / z3, u = a3 * iz3, rho = z * u, h = 0.5 * iz3;
+      const double z3 = z + a3, iz3 = 1.0 / z3, u = a3 * iz3, rho = ratio(z * a3, z3, iz3), h = 0.5 * iz3;
       double pref;      // of the moments, the image's exponential apart
       if (OP == OLC_OP_NUCLEAR) {
         pref = -pt.nuc_charge * 2.0 * (kPi * iz3) * expAB;
