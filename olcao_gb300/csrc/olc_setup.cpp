@@ -17,6 +17,9 @@
 #include <cmath>
 #include <cstring>
 #include <functional>
+#include <map>
+#include <memory>
+#include <utility>
 
 #include "olc_common.h"
 
@@ -444,65 +447,77 @@ int build_system(olc_context* ctx, const olc_system_t* s) {
   // ---- alpha-pair items grouped by (l1, l2) class -------------------------
   // The pairs of two types, the most diffuse first: the third-centre radius
   // falls with a1 + a2, so neighbouring threads of the primitive kernels sum
-  // about the same number of images.
+  // about the same number of images.  Tasks between the same two of a type pair's
+  // radii have the same items: each such list is made once, by class, when the first
+  // of its tasks asks for it.  Types that differ in their radial functions alone
+  // share all of it.
   struct AlphaPair {
     double dist, sum;
     int cls;
     int32_t ab;
   };
-  std::vector<std::vector<AlphaPair>> typePairs((size_t)s->num_atom_types * s->num_atom_types);
-  for (int x = 0; x < s->num_atom_types; ++x)
-    for (int y = 0; y < s->num_atom_types; ++y) {
-      const DevType &t1 = ctx->htypes[x], &t2 = ctx->htypes[y];
-      auto& tp = typePairs[(size_t)x * s->num_atom_types + y];
-      for (int a1 = 0; a1 < t1.nalpha; ++a1) {
-        // the row of a1 ends at its first pair out of reach: every pair is held to the
-        // smallest radius up to it (past the exponents of an element's first type
-        // the radius is not defined and the table gives infinity)
-        double dist = HUGE_VAL;
-        for (int a2 = 0; a2 < t2.nalpha; ++a2) {
-          const double d = alphaDist(a1, a2, t1.element, t2.element);
-          if (d < dist) dist = d;
-          tp.push_back({dist, t1.alphas[a1] + t2.alphas[a2], t1.lmax_alpha[a1] * (kMaxL + 1) + t2.lmax_alpha[a2],
-                        a1 | (a2 << 8)});
-        }
-      }
-      std::stable_sort(tp.begin(), tp.end(), [](const AlphaPair& p, const AlphaPair& q) { return p.sum < q.sum; });
-    }
-  // Tasks between the same two of a type pair's radii have the same items: each such
-  // list is made once, by class, when the first of its tasks asks for it.
   struct Reach {
-    std::vector<double> radius;                                   // descending, each once
-    std::vector<std::array<std::vector<int32_t>, kNumClasses>> ab;   // of the pairs with dist >= radius[q]
+    std::vector<AlphaPair> pairs;
+    std::vector<double> radius;                                           // descending, each once
+    std::vector<std::unique_ptr<std::array<std::vector<int32_t>, kNumClasses>>> ab;   // of dist >= radius[q]
   };
-  std::vector<Reach> reach(typePairs.size());
-  for (size_t x = 0; x < typePairs.size(); ++x) {
-    Reach& r = reach[x];
-    for (const AlphaPair& e : typePairs[x]) r.radius.push_back(e.dist);
+  std::vector<int> kind(s->num_atom_types);
+  for (int x = 0; x < s->num_atom_types; ++x) {
+    const DevType& t = ctx->htypes[x];
+    for (kind[x] = 0; kind[x] < x; ++kind[x]) {
+      const DevType& u = ctx->htypes[kind[x]];
+      if (u.element == t.element && u.nalpha == t.nalpha && std::equal(t.alphas, t.alphas + t.nalpha, u.alphas) &&
+          std::equal(t.lmax_alpha, t.lmax_alpha + t.nalpha, u.lmax_alpha))
+        break;
+    }
+  }
+  std::map<std::pair<int, int>, Reach> reaches;
+  auto make_reach = [&](const DevType& t1, const DevType& t2, Reach& r) {
+    for (int a1 = 0; a1 < t1.nalpha; ++a1) {
+      // the row of a1 ends at its first pair out of reach: every pair is held to the
+      // smallest radius up to it (past the exponents of an element's first type
+      // the radius is not defined and the table gives infinity)
+      double dist = HUGE_VAL;
+      for (int a2 = 0; a2 < t2.nalpha; ++a2) {
+        const double d = alphaDist(a1, a2, t1.element, t2.element);
+        if (d < dist) dist = d;
+        r.pairs.push_back({dist, t1.alphas[a1] + t2.alphas[a2], t1.lmax_alpha[a1] * (kMaxL + 1) + t2.lmax_alpha[a2],
+                           a1 | (a2 << 8)});
+        r.radius.push_back(dist);
+      }
+    }
+    std::stable_sort(r.pairs.begin(), r.pairs.end(),
+                     [](const AlphaPair& p, const AlphaPair& q) { return p.sum < q.sum; });
     std::sort(r.radius.begin(), r.radius.end(), std::greater<double>());
     r.radius.erase(std::unique(r.radius.begin(), r.radius.end()), r.radius.end());
     r.ab.resize(r.radius.size());
-  }
+  };
   std::vector<int32_t> itTask[kNumClasses], itAB[kNumClasses], itStart[kNumClasses];
   for (int c = 0; c < kNumClasses; ++c) itStart[c].assign(ntasks + 1, 0);
+  int pair = -1;
+  Reach* reach = nullptr;
   for (int q = 0; q < ntasks; ++q) {
     const DevTask& tk = ctx->htasks[q];
-    const DevPair& p = ctx->hpairs[tk.pair];
     for (int c = 0; c < kNumClasses; ++c) itStart[c][q] = (int32_t)itTask[c].size();
-    const size_t x = (size_t)siteType[p.i] * s->num_atom_types + siteType[p.j];
-    Reach& r = reach[x];
-    const size_t in = std::partition_point(r.radius.begin(), r.radius.end(),
-                                           [&](double d) { return !(d < tk.sep); }) - r.radius.begin();
+    if (tk.pair != pair) {
+      pair = tk.pair;
+      const DevPair& p = ctx->hpairs[pair];
+      const int x = kind[siteType[p.i]], y = kind[siteType[p.j]];
+      reach = &reaches[{x, y}];
+      if (reach->pairs.empty()) make_reach(ctx->htypes[x], ctx->htypes[y], *reach);
+    }
+    const size_t in = std::partition_point(reach->radius.begin(), reach->radius.end(),
+                                           [&](double d) { return !(d < tk.sep); }) - reach->radius.begin();
     if (in == 0) continue;
-    auto& list = r.ab[in - 1];
-    bool made = false;
-    for (const auto& l : list) made = made || !l.empty();
-    if (!made)
-      for (const AlphaPair& e : typePairs[x])
-        if (e.dist >= r.radius[in - 1]) list[e.cls].push_back(e.ab);
+    auto& list = reach->ab[in - 1];
+    if (!list) {
+      list = std::make_unique<std::array<std::vector<int32_t>, kNumClasses>>();
+      for (const AlphaPair& e : reach->pairs)
+        if (e.dist >= reach->radius[in - 1]) (*list)[e.cls].push_back(e.ab);
+    }
     for (int c = 0; c < kNumClasses; ++c) {
-      itTask[c].insert(itTask[c].end(), list[c].size(), q);
-      itAB[c].insert(itAB[c].end(), list[c].begin(), list[c].end());
+      itTask[c].insert(itTask[c].end(), (*list)[c].size(), q);
+      itAB[c].insert(itAB[c].end(), (*list)[c].begin(), (*list)[c].end());
     }
   }
   for (int c = 0; c < kNumClasses; ++c) itStart[c][ntasks] = (int32_t)itTask[c].size();
