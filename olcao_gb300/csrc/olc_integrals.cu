@@ -178,8 +178,9 @@ struct ContractArgs {
 };
 
 // One CTA per (task, kContractCols states of the second atom).  The FP64 pipe
-// bounds the contraction, so it runs in two steps, as pairXBasisFn2 and
-// multWithBasisFn1 do: T(a1, lm1; m2) = sum_a2 c2(a2, m2) sh(a1, a2; lm1, lm2)
+// would bound one sum per element, so it runs in two steps, as pairXBasisFn2 and
+// multWithBasisFn1 do (the pipe is then 39 % busy at 64 silicon atoms, and the loads
+// of the primitive blocks bound it): T(a1, lm1; m2) = sum_a2 c2(a2, m2) sh(a1, a2; lm1, lm2)
 // in shared memory, then block(m1, m2) = sum_a1 c1(a1, m1) T(a1, lm(m1); m2)
 // -- about 9 n_a^2 M2 + n_a M1 M2 multiply-adds where one sum per element over
 // all alpha pairs costs 3 n_a^2 M1 M2 operations.  Per operator: two-atom cell

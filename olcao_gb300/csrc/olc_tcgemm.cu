@@ -205,9 +205,10 @@ inline int smem_total(int mode, int slots_a, int slots_b) {
 // for half of its pairs, the copies run at the 5.4 TB/s that all SMs together
 // reach, and what is left of the 34 pairs hides about a third of them.  In the
 // f32 mode the copies' latency at the K-steps' ends.  Measured: FP64-accurate
-// product of order 1248 1025 -> 818 us, FP32-accurate one with its slices 133 -> 125
-// us; a mixed pass over 64 matrices of order 832: FP64-accurate products
-// 22.7 -> 19 ms, FP32-accurate ones (as then formed) 18.5 -> 14.2 ms.
+// product of order 1248 1025 -> 818 us; FP32-accurate ones with their slices 75 -> 72
+// (order 832, the kernel alone 55 -> 60) and 362 -> 325 us (2000, 274 -> 277); a mixed
+// pass over 64 matrices of order 832: FP64-accurate products 22.7 -> 18.8 ms,
+// FP32-accurate ones (as then formed) 18.5 -> 14.2 ms, now 11.5.
 // MODE 0 (fixed): BN = 128, four accumulators of 128 columns, int64 drains,
 //   FP64 complex output.  Epilogue warp w owns TMEM lanes 32 (w % 4) .. +31
 //   and columns 32 (w / 4) .. +31 of the tile (16 complex columns).
